@@ -3,12 +3,13 @@
 // Kernel selection by size replaces the reference's compile-time tuning tables
 // (library/src/include/ideal_sizes.hpp:208-240 getrf, :166-180 potrf;
 // roclapack_getf2.hpp:181-276 select_spkernel): the CTA LU configuration comes from the
-// run-time tuning table (tuning.h) when it has an entry, else from the built-in choice.
+// run-time tuning table (tuning.h) when it has an entry, else the blocked LU (lu_blk.cuh).
 #include <algorithm>
 
 #include "chol.cuh"
 #include "launch.h"
 #include "logger.h"
+#include "lu_blk.h"
 #include "lu_cta.cuh"
 #include "lu_small.cuh"
 #include "trsv.cuh"
@@ -229,31 +230,21 @@ static rocblas_status getrf_dispatch(cudaStream_t s, int m, int n, Batch<T> A, i
         if(ran)
             return st;
     }
-    // built-in choice (used when no tuning table is installed)
-    if(m <= 64)
-        return run_getrf_cta<T, 64, 1, 32, PIVOT, TC>(s, m, n, A, lda, ipiv, sP, info, bc,
-                                                   g, 0, 0);
-    if(m <= 128)
-        return run_getrf_cta<T, 128, 1, 32, PIVOT, TC>(s, m, n, A, lda, ipiv, sP, info, bc,
-                                                   g, 0, 0);
-    // FP32: 128-thread CTAs with two rows per thread (three CTAs per SM); FP64 keeps
-    // 256 threads (its two-row panel would not fit the register budget)
-    if(sizeof(T) == 4 && m <= 256)
-        return run_getrf_cta<T, 128, 2, 32, PIVOT, TC>(s, m, n, A, lda, ipiv, sP, info, bc,
-                                                   g, 0, 0);
-    if(m <= 256)
-        return run_getrf_cta<T, 256, 1, 32, PIVOT, TC>(s, m, n, A, lda, ipiv, sP, info, bc,
-                                                   g, 0, 0);
-    if(m <= 512)
-        return run_getrf_cta<T, 256, 2, 16, PIVOT, TC>(s, m, n, A, lda, ipiv, sP, info, bc,
-                                                   g, 0, 0);
-    if(m <= 1024)
-        return run_getrf_cta<T, 256, 4, 8, PIVOT, TC>(s, m, n, A, lda, ipiv, sP, info, bc,
-                                                   g, 0, 0);
-    if(m <= MAX_CTA_ROWS)
-        return run_getrf_cta<T, 256, 8, 4, PIVOT, TC>(s, m, n, A, lda, ipiv, sP, info, bc,
-                                                   g, 0, 0);
-    return rocblas_status_not_implemented;
+    // Without an entry: the blocked LU in separate launches, for every m > 32.  Measured against
+    // the one-launch CTA kernels with their tuned entries (getrf alone, ms, blocked / CTA): FP64
+    // n = 64 x 16384 1.06 / 1.65, n = 128 x 8192 2.53 / 3.20, n = 256 x 2048 3.53 / 3.78, n = 512
+    // x 592 6.95 / 7.12, n = 2048 x 16 10.3 / 161; FP32 n = 501 x 200 2.09 / 2.93; split TF32
+    // n = 256 x 2048 2.00 / 2.23.  The CTA kernels remain for tables that name them.
+    LuBatch<T> L{};
+    L.A = A;
+    L.m = m;
+    L.n = n;
+    L.lda = lda;
+    L.ipiv = ipiv;
+    L.strideP = sP;
+    L.info = info;
+    L.gate = g;
+    return launch_lu_blk<T>(s, L, m, n, bc, PIVOT, TC);
 }
 
 template <typename T>

@@ -20,24 +20,11 @@
 #include "lu_cta.cuh"
 #include "lu_small.cuh"
 #include "trsv.cuh"
+#include "vbatched.h"
 
 namespace rsb {
 
-constexpr int VB_SMALL = 32;   // members with n <= VB_SMALL use the warp path
 constexpr int VB_WARPS = 8;    // CTA = 8 warps = 256 threads
-
-struct VbArgs
-{
-    int bc, max_n, max_nrhs, mode; // mode: 0 gesv, 1 getrf, 2 getrs
-    const int* n;
-    const int* nrhs;
-    const int* lda;
-    const int* ldb;
-    int* const* ipiv;
-    int* info;
-    int* order;    // [bc]
-    int* counters; // [0] big cursor, [1] small cursor, [2] number of big members
-};
 
 __global__ void __launch_bounds__(1024) vb_plan_kernel(VbArgs v)
 {
@@ -76,21 +63,6 @@ __global__ void __launch_bounds__(1024) vb_plan_kernel(VbArgs v)
         v.order[atomicAdd(&hist[bucket(b)], 1)] = b;
 }
 
-template <typename T>
-__device__ __forceinline__ bool vb_valid(const VbArgs& v, int b)
-{
-    const int n = v.n[b];
-    if(n < 0 || n > v.max_n || v.lda[b] < max(1, n))
-        return false;
-    if(v.mode != 1)
-    {
-        const int r = v.nrhs[b];
-        if(r < 0 || r > v.max_nrhs || v.ldb[b] < max(1, n))
-            return false;
-    }
-    return true;
-}
-
 template <typename T, int NT, int R, int JB, int TN>
 __global__ void __launch_bounds__(NT, R * JB > 32 ? 1 : 2)
     vb_persistent_kernel(VbArgs v, T* const* A, T* const* B, int cw, int fold)
@@ -112,7 +84,7 @@ __global__ void __launch_bounds__(NT, R * JB > 32 ? 1 : 2)
         if(t >= nbig)
             break;
         const int b = v.order[t];
-        if(!vb_valid<T>(v, b))
+        if(!vb_valid(v, b))
         {
             if(tid == 0 && v.mode != 2)
                 v.info[b] = -1;
@@ -154,7 +126,7 @@ __global__ void __launch_bounds__(NT, R * JB > 32 ? 1 : 2)
         if(t < v.bc)
         {
             const int b = v.order[t];
-            if(!vb_valid<T>(v, b))
+            if(!vb_valid(v, b))
             {
                 if((tid & 31) == 0 && v.mode != 2)
                     v.info[b] = -1;
