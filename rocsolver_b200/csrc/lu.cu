@@ -7,6 +7,7 @@
 #include <algorithm>
 
 #include "chol.cuh"
+#include "chol_blk.cuh"
 #include "launch.h"
 #include "logger.h"
 #include "lu_blk.h"
@@ -371,28 +372,53 @@ rocblas_status launch_gesv(cudaStream_t s, int n, int nrhs, Batch<T> A, int lda,
 }
 
 // ------------------------------------------------------------------------------ potrf
-template <typename T, int NT, int R, int JB, int TN>
-static rocblas_status run_potrf(cudaStream_t s, int upper, int n, Batch<T> A, int lda,
-                                int* info, int bc)
+template <typename T, int N>
+static rocblas_status run_potrf_reg(cudaStream_t s, int upper, int n, Batch<T> A, int lda,
+                                    int* info, int bc, int j0 = 0)
 {
-    size_t smem = sizeof(T) * 2 * JB;
-    if(n > JB)
-        smem += sizeof(T) * (size_t)R * NT * (JB + 1);
-    auto k = potrf_cta_kernel<T, NT, R, JB, TN>;
-    if(!set_smem(k, smem))
-        return rocblas_status_internal_error;
-    RSB_LOG_KERNEL("potrf_cta_kernel");
-    k<<<bc, NT, smem, s>>>(upper, n, A, lda, info);
+    RSB_LOG_KERNEL("potrf_reg_kernel");
+    if(upper)
+        potrf_reg_kernel<T, N, true><<<bc, N, 0, s>>>(n, A, lda, info, j0);
+    else
+        potrf_reg_kernel<T, N, false><<<bc, N, 0, s>>>(n, A, lda, info, j0);
     return launch_status();
 }
 
-template <typename T, int N>
-static rocblas_status run_potrf_reg(cudaStream_t s, int upper, int n, Batch<T> A, int lda,
-                                    int* info, int bc)
+// n > 64: steps of 64 columns (chol_blk.cuh)
+template <typename T, bool UPPER>
+static rocblas_status run_potrf_blk(cudaStream_t s, int n, Batch<T> A, int lda, int* info, int bc)
 {
-    RSB_LOG_KERNEL("potrf_reg_kernel");
-    potrf_reg_kernel<T, N><<<bc, N, 0, s>>>(upper, n, A, lda, info);
-    return launch_status();
+    constexpr int NB = BLK_NB;
+    if(!set_smem(potrf_trsm_kernel<T, UPPER>, sizeof(CholTrsmSmem<T>))
+       || !set_smem(potrf_syrk_kernel<T, UPPER>, sizeof(GemmSmem<T>)))
+        return rocblas_status_internal_error;
+    for(int j0 = 0; j0 < n; j0 += NB)
+    {
+        const int jb = std::min(NB, n - j0), below = n - j0 - jb;
+        const rocblas_status st = jb <= 32
+                                      ? run_potrf_reg<T, 32>(s, UPPER, jb, A, lda, info, bc, j0)
+                                      : run_potrf_reg<T, 64>(s, UPPER, jb, A, lda, info, bc, j0);
+        if(st != rocblas_status_success || below <= 0)
+            return st;
+        const int chunks = (below + CHOL_CW - 1) / CHOL_CW, t = (below + 63) / 64;
+        const int tiles = t * (t + 1) / 2;
+        {
+            RSB_LOG_KERNEL("potrf_trsm_kernel");
+            potrf_trsm_kernel<T, UPPER><<<(unsigned)((int64_t)bc * chunks), CHOL_NT,
+                                          sizeof(CholTrsmSmem<T>), s>>>(n, A, lda, info, j0,
+                                                                        chunks);
+        }
+        if(launch_status() != rocblas_status_success)
+            return rocblas_status_internal_error;
+        {
+            RSB_LOG_KERNEL("potrf_syrk_kernel");
+            potrf_syrk_kernel<T, UPPER><<<(unsigned)((int64_t)bc * tiles), 128,
+                                          sizeof(GemmSmem<T>), s>>>(n, A, lda, info, j0, tiles);
+        }
+        if(launch_status() != rocblas_status_success)
+            return rocblas_status_internal_error;
+    }
+    return rocblas_status_success;
 }
 
 template <typename T>
@@ -403,15 +429,10 @@ rocblas_status launch_potrf(cudaStream_t s, int upper, int n, Batch<T> A, int ld
         return run_potrf_reg<T, 32>(s, upper, n, A, lda, info, bc);
     if(n <= 64)
         return run_potrf_reg<T, 64>(s, upper, n, A, lda, info, bc);
-    if(n <= 256)
-        return run_potrf<T, 256, 1, 32, 8>(s, upper, n, A, lda, info, bc);
-    if(n <= 512)
-        return run_potrf<T, 256, 2, 16, 8>(s, upper, n, A, lda, info, bc);
-    if(n <= 1024)
-        return run_potrf<T, 256, 4, 8, 4>(s, upper, n, A, lda, info, bc);
-    if(n <= MAX_CTA_ROWS)
-        return run_potrf<T, 256, 8, 4, 4>(s, upper, n, A, lda, info, bc);
-    return rocblas_status_not_implemented;
+    if(n > MAX_CTA_ROWS)
+        return rocblas_status_not_implemented;
+    return upper ? run_potrf_blk<T, true>(s, n, A, lda, info, bc)
+                 : run_potrf_blk<T, false>(s, n, A, lda, info, bc);
 }
 
 template <typename T, int NT, int NRC>

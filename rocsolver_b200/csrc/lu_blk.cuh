@@ -999,7 +999,7 @@ __global__ void __launch_bounds__(TRSM_NT, sizeof(T) == 8 ? 3 : 5)
 }
 
 // ---------------------------------------------------------------------------- A22
-// Warp tiles of 32 x 32 on operands sA[k][row] and sB (FP64: [col][k], else [k][col]).
+// Warp tiles of 32 x 32 on operands sA[k][row] and sB ([col][k] for B_BY_COL, else [k][col]).
 constexpr int GEMM_LD = 68; // = 4 mod 32 (32-bit) and 4 mod 16 (64-bit): no bank conflicts
 
 template <typename T, bool TC>
@@ -1010,6 +1010,7 @@ struct GemmTile<double, false>
 {
     double acc[4][4][2];
     static constexpr bool B_BY_COL = true;
+    template <bool BY_COL = true>
     __device__ __forceinline__ void mma(const double* sA, const double* sB, int r0, int c0, int kk)
     {
         const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
@@ -1022,7 +1023,8 @@ struct GemmTile<double, false>
                 a[i] = sA[(k0 + q) * GEMM_LD + r0 + i * 8 + g];
 #pragma unroll
             for(int i = 0; i < 4; ++i)
-                b[i] = sB[(c0 + i * 8 + g) * GEMM_LD + k0 + q];
+                b[i] = BY_COL ? sB[(c0 + i * 8 + g) * GEMM_LD + k0 + q]
+                              : sB[(k0 + q) * GEMM_LD + c0 + i * 8 + g];
 #pragma unroll
             for(int i = 0; i < 4; ++i)
 #pragma unroll
@@ -1052,6 +1054,7 @@ struct GemmTile<float, false>
 {
     float2 acc[4][4]; // rows rg*4 + i, columns cg*8 + 2p + {0, 1}
     static constexpr bool B_BY_COL = false;
+    template <bool BY_COL = false>
     __device__ __forceinline__ void mma(const float* sA, const float* sB, int r0, int c0, int kk)
     {
         const int lane = threadIdx.x & 31, rg = lane & 7, cg = lane >> 3;
