@@ -3,7 +3,8 @@
 // Kernel selection by size replaces the reference's compile-time tuning tables
 // (library/src/include/ideal_sizes.hpp:208-240 getrf, :166-180 potrf;
 // roclapack_getf2.hpp:181-276 select_spkernel): the CTA LU configuration comes from the
-// run-time tuning table (tuning.h) when it has an entry, else the blocked LU (lu_blk.cuh).
+// run-time tuning table (tuning.h) when it has an entry, else from the built-in choice
+// between them and the blocked LU (lu_blk.cuh).
 #include <algorithm>
 
 #include "chol.cuh"
@@ -231,11 +232,33 @@ static rocblas_status getrf_dispatch(cudaStream_t s, int m, int n, Batch<T> A, i
         if(ran)
             return st;
     }
-    // Without an entry: the blocked LU in separate launches, for every m > 32.  Measured against
-    // the one-launch CTA kernels with their tuned entries (getrf alone, ms, blocked / CTA): FP64
-    // n = 64 x 16384 1.06 / 1.65, n = 128 x 8192 2.53 / 3.20, n = 256 x 2048 3.53 / 3.78, n = 512
-    // x 592 6.95 / 7.12, n = 2048 x 16 10.3 / 161; FP32 n = 501 x 200 2.09 / 2.93; split TF32
-    // n = 256 x 2048 2.00 / 2.23.  The CTA kernels remain for tables that name them.
+    // Without an entry, FP64 up to 512 rows: the one-launch CTA kernels.  The factors feed
+    // inverses and adjoints of matrices whose condition nothing bounds (uniform + 4 I, 16384
+    // members of n = 64, hold one of 1e7 now and then), where another order of rounding shows:
+    // with the blocked LU these outputs moved by 1e-9 to 4e-9 (relative, 2-norm) in one of ten
+    // to one of four batches of n = 64 .. 256, beyond the 5e-10 that such solves are held to,
+    // at the same error against 64-bit results.  The blocked LU is no clear gain there either
+    // (getrf alone, ms, blocked / CTA): n = 64 x 16384 1.06 / 1.63, n = 65 x 16384 3.08 / 2.64,
+    // n = 128 x 8178 2.52 / 3.04, n = 129 x 8052 5.65 / 4.52, n = 200 x 3350 4.80 / 4.06,
+    // n = 256 x 2044 3.52 / 3.79, n = 512 x 592 6.95 / 7.12.
+    if constexpr(sizeof(T) == 8)
+    {
+        if(m <= 64)
+            return run_getrf_cta<T, 64, 1, 32, PIVOT, TC>(s, m, n, A, lda, ipiv, sP, info, bc, g,
+                                                          0, 0);
+        if(m <= 128)
+            return run_getrf_cta<T, 128, 1, 32, PIVOT, TC>(s, m, n, A, lda, ipiv, sP, info, bc,
+                                                           g, 0, 0);
+        if(m <= 256)
+            return run_getrf_cta<T, 256, 1, 32, PIVOT, TC>(s, m, n, A, lda, ipiv, sP, info, bc,
+                                                           g, 0, 0);
+        if(m <= 512)
+            return run_getrf_cta<T, 256, 2, 16, PIVOT, TC>(s, m, n, A, lda, ipiv, sP, info, bc,
+                                                           g, 0, 0);
+    }
+    // The rest: the blocked LU in separate launches.  Measured against the CTA kernels with
+    // their tuned entries (getrf alone, ms, blocked / CTA): FP64 n = 2048 x 16 10.3 / 161; FP32
+    // n = 501 x 200 2.09 / 2.93; split TF32 n = 256 x 2048 2.00 / 2.23.
     LuBatch<T> L{};
     L.A = A;
     L.m = m;

@@ -121,6 +121,24 @@ def test_getrf_uniform_square(handle, n, dtype):
             assert be / (n * eps_of(dtype)) < 10
 
 
+@pytest.mark.parametrize("n", [33, 64, 65, 128, 129, 256, 300, 512])
+def test_dgetrf_rounds_as_the_cta_kernel(handle, n):
+    """The FP64 factors of the shipped configuration are, bit for bit, those of the CTA kernel
+    with panels of 32 columns: an inverse from them amplifies any other order of rounding by the
+    condition of the worst member, which programs compare between runs and versions."""
+    A = uniform_general(n, n, 3, seed=31 * n) + 4 * np.eye(n)
+    LU, ipiv, info, _ = gpu_getrf(handle, A)
+    old = rs.tuning_table()
+    try:
+        assert rs.set_tuning_table("getrf d 512 256 2 32 64 0\n") == rs.SUCCESS
+        LU2, ipiv2, info2, _ = gpu_getrf(handle, A)
+    finally:
+        assert rs.set_tuning_table(old) == rs.SUCCESS
+    np.testing.assert_array_equal(ipiv, ipiv2)
+    np.testing.assert_array_equal(info, info2)
+    np.testing.assert_array_equal(LU, LU2)
+
+
 @pytest.mark.parametrize("n", [16, 33, 64, 100, 128, 200, 256, 300, 512, 1024])
 def test_sgetrf_tf32(handle, n):
     """rocsolver_sgetrf_tf32_strided_batched (split-TF32 tensor-core trailing updates, the
