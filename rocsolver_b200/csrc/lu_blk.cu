@@ -2,6 +2,7 @@
 #include "lu_blk.h"
 
 #include <algorithm>
+#include <cstdlib>
 
 #include "logger.h"
 
@@ -19,6 +20,17 @@ rocblas_status launched()
 {
     return cudaGetLastError() == cudaSuccess ? rocblas_status_success
                                              : rocblas_status_internal_error;
+}
+
+// polls after which a wait between the CTAs of a cluster gives up; the bounds-checked build
+// takes another limit from the environment, so that a test can see the waits run out
+int cluster_wait_limit()
+{
+#ifdef RSB_BOUNDS_CHECK
+    if(const char* e = std::getenv("ROCSOLVER_B200_CLUSTER_WAIT"))
+        return std::atoi(e);
+#endif
+    return CLUSTER_WAIT_LIMIT;
 }
 
 template <typename T, int S, bool PIVOT, bool CL>
@@ -42,7 +54,7 @@ rocblas_status panel(cudaStream_t s, const LuBatch<T>& L, int j0, int lo, int hi
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = CL ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k, L, j0, lo, hi) == cudaSuccess
+    return cudaLaunchKernelEx(&cfg, k, L, j0, lo, hi, cluster_wait_limit()) == cudaSuccess
                ? launched()
                : rocblas_status_internal_error;
 }

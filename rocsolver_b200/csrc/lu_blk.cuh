@@ -73,6 +73,14 @@ __device__ __forceinline__ bool lu_member(const LuBatch<T>& L, int64_t i, LuMemb
     return true;
 }
 
+// A panel of this member (one of more than 256 rows, in a cluster) gave up a wait: its factors
+// are not valid, its pivots are the identity, and the launches that follow leave it alone.
+template <typename T>
+__device__ __forceinline__ bool lu_gave_up(const LuBatch<T>& L, const LuMember<T>& M)
+{
+    return L.m > 256 && *M.info == INT_MIN;
+}
+
 // ---------------------------------------------------------------------------- PTX helpers
 __device__ __forceinline__ void cluster_sync_all()
 {
@@ -116,13 +124,21 @@ __device__ __forceinline__ void mbar_expect(uint64_t* b, uint32_t bytes)
                  "r"(bytes)
                  : "memory");
 }
-// wait for the phase with this parity; false when it has not come after CLUSTER_WAIT_LIMIT
-// polls of a microsecond
+// stands in for bytes that will not be sent
+__device__ __forceinline__ void mbar_complete(uint64_t* b, uint32_t bytes)
+{
+    asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;\n" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(b))),
+                 "r"(bytes)
+                 : "memory");
+}
+// wait for the phase with this parity; false when it has not come after limit polls of a
+// microsecond
 constexpr int CLUSTER_WAIT_LIMIT = 1 << 20;
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* b, uint32_t parity)
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* b, uint32_t parity, int limit)
 {
     const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(b));
-    for(int i = 0; i < CLUSTER_WAIT_LIMIT; ++i)
+    for(int i = 0; i < limit; ++i)
     {
         uint32_t ok;
         asm volatile("{\n\t.reg .pred p;\n\t"
@@ -147,6 +163,10 @@ __device__ __forceinline__ float ld_cluster(uint32_t addr, float)
     float v;
     asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(addr) : "memory");
     return v;
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, int v)
+{
+    asm volatile("st.shared::cluster.s32 [%0], %1;\n" ::"r"(addr), "r"(v) : "memory");
 }
 template <int NT>
 __device__ __forceinline__ void cta_bar()
@@ -238,6 +258,8 @@ struct PanelSmem
     int label[32 * S];
     int piv[NB];                    // label of each column's pivot row
     int owner[8], slot[8];          // rank and slot of each pivot row of the group
+    int mysent[2], sent[16];        // (cluster) columns whose record was sent: own, [rank, warp]
+    int failed;                     // (cluster) a wait of this CTA ran out
 };
 
 // State of the warp that factors the groups
@@ -247,7 +269,7 @@ struct PanelLabels
     int lab[S];     // position of each row (row lane + 32 s), -1: no row
     int inf;        // first zero pivot
     uint32_t phase; // (cluster) parity bits of the two barriers
-    bool failed;
+    bool failed;    // (cluster) a wait ran out
 };
 
 // Columns c0 .. c0+gb-1 (gb <= 8) of the panel by FW warps: lane i of warp f holds rows i,
@@ -262,12 +284,15 @@ struct PanelLabels
 // current column is always entry 0): unrolled, its code did not stay in the instruction
 // cache.  A pivot row's remaining entries go to its slot when it is found; what the registers
 // of a finished row hold after that is not used.
+// A cluster wait that runs out (wait_limit polls) ends the warp's part in the panel: it sends
+// and reads no further record, so that the other CTAs' waits run out in turn, and leaves the
+// group's rows and slots in range for the threads that go on to the barriers.
 // Time of one 64-column FP64 panel alone on an SM: 64 rows (S = 2) 36 us, 128 rows 33 us; 256
 // rows took 58 us with one warp of 8 rows a lane, which is why they have two.
 template <typename T, int NB, int SC, bool PIVOT, bool CL>
 __device__ __forceinline__ void panel_group(PanelSmem<T, NB, SC>& sm,
                                             PanelLabels<PanelShape<T, SC>::FS>& st, int f, int c0,
-                                            int gb, int j0, int rank, int nrank)
+                                            int gb, int j0, int rank, int nrank, int wait_limit)
 {
     constexpr int S = PanelShape<T, SC>::FS, FW = PanelShape<T, SC>::FW;
     using K = typename KeyOf<T>::type;
@@ -280,9 +305,12 @@ __device__ __forceinline__ void panel_group(PanelSmem<T, NB, SC>& sm,
 #pragma unroll
         for(int k = 0; k < 8; ++k)
             x[s][k] = sm.P[c0 + k][f * 32 * S + lane + 32 * s];
+    int k = 0;
 #pragma unroll 1
-    for(int k = 0; k < gb; ++k)
+    for(; k < gb; ++k)
     {
+        if(CL && st.failed)
+            break;
         const int c = c0 + k;
         // (selections, no branches: a divergent branch per row costs more than the row)
         uint32_t hv[S];
@@ -378,9 +406,16 @@ __device__ __forceinline__ void panel_group(PanelSmem<T, NB, SC>& sm,
                          reinterpret_cast<const uint4*>(&sm.mine[f])[q],
                          map_rank(&sm.mbar[k & 1], to));
             }
-            if(!st.failed && !mbar_wait_cluster(&sm.mbar[k & 1], (st.phase >> (k & 1)) & 1u))
-                st.failed = true;
-            st.failed = __any_sync(full, st.failed);
+            const bool came =
+                mbar_wait_cluster(&sm.mbar[k & 1], (st.phase >> (k & 1)) & 1u, wait_limit);
+            st.failed = !__all_sync(full, came);
+            if(st.failed)
+            {
+                // the records of this column may be unwritten
+                if(lane == 0)
+                    sm.mysent[f] = c + 1;
+                break;
+            }
             st.phase ^= 1u << (k & 1);
             const PanelRec<T>& rl = sm.rec[k & 1][lane & 15];
             const bool in = lane < nrec && rl.label != INT_MAX;
@@ -454,6 +489,15 @@ __device__ __forceinline__ void panel_group(PanelSmem<T, NB, SC>& sm,
             sm.owner[k] = w;
             sm.slot[k] = wslot;
             sm.piv[c] = wl;
+        }
+    }
+    if(CL && st.failed && f == 0 && lane < 8)
+    {
+        if(lane >= k)
+        {
+            sm.owner[lane] = rank;
+            sm.slot[lane] = 0;
+            sm.piv[c0 + lane] = c0 + lane;
         }
     }
     // the pivot rows' multipliers within the group, for U of the columns right of it
@@ -611,7 +655,7 @@ __global__ void __launch_bounds__(PanelShape<T, S>::NT,
                                   S <= 2   ? (sizeof(T) == 8 ? 4 : 6)
                                   : S <= 4 ? (sizeof(T) == 8 ? 2 : 3)
                                            : (sizeof(T) == 8 || CL ? 1 : 2))
-    lu_panel_kernel(LuBatch<T> L, int j0, int rows_lo, int rows_hi)
+    lu_panel_kernel(LuBatch<T> L, int j0, int rows_lo, int rows_hi, int wait_limit)
 {
     using SH = PanelShape<T, S>;
     constexpr int RT = SH::RT, NT = SH::NT, NC = NB / 8 - 1;
@@ -624,7 +668,7 @@ __global__ void __launch_bounds__(PanelShape<T, S>::NT,
         rank = cluster_rank();
     }
     LuMember<T> M;
-    if(!lu_member(L, blockIdx.x / nrank, M))
+    if(!lu_member(L, blockIdx.x / nrank, M) || (j0 > 0 && lu_gave_up(L, M)))
         return;
     const int mn = min(M.m, M.n), mp = M.m - j0;
     if(j0 >= mn || mp <= rows_lo || mp > rows_hi)
@@ -640,6 +684,8 @@ __global__ void __launch_bounds__(PanelShape<T, S>::NT,
         {
             mbar_init_cluster(&sm.mbar[0], 1);
             mbar_init_cluster(&sm.mbar[1], 1);
+            sm.failed = 0;
+            sm.mysent[0] = sm.mysent[1] = jb;
         }
         cluster_sync_all(); // every CTA's barriers are ready before a candidate is sent
     }
@@ -755,7 +801,7 @@ __global__ void __launch_bounds__(PanelShape<T, S>::NT,
         {
             cta_bar<NT>();
             panel_group<T, NB, S, PIVOT, CL>(sm, lb, f, 8 * gi, min(8, jb - 8 * gi), j0, rank,
-                                              nrank);
+                                              nrank, wait_limit);
             cta_bar<NT>();
             if(gi + 1 < ngroup)
             {
@@ -780,14 +826,19 @@ __global__ void __launch_bounds__(PanelShape<T, S>::NT,
             for(int c = lane; c < jb; c += 32)
                 M.piv[j0 + c] = j0 + sm.piv[c] + 1;
         }
-        if(lane == 0 && lb.failed)
-            *M.info = INT_MIN; // a cluster wait ran out: the results are not valid
-        else if(lane == 0 && rank == 0 && f == 0 && (j0 == 0 || (lb.inf != 0 && *M.info == 0)))
+        if(lane == 0 && rank == 0 && f == 0 && (j0 == 0 || (lb.inf != 0 && *M.info == 0)))
             *M.info = lb.inf;
+        if(CL)
+        {
+            if(lane == 0 && lb.failed)
+                sm.failed = 1;
+            if(lane < nrank)
+                st_cluster(map_rank(&sm.sent[rank * SH::FW + f], lane), sm.mysent[f]);
+        }
     }
     cta_bar<NT>();
     // finished columns to their final positions (all of the panel was read at the start)
-    if(tid < mc)
+    if(tid < mc && !(CL && sm.failed))
     {
         const int pos = sm.label[tid];
 #pragma unroll 8
@@ -795,7 +846,40 @@ __global__ void __launch_bounds__(PanelShape<T, S>::NT,
             RSB_AT(M.a, j0 + pos, j0 + k, M.lda, M.m, M.n) = sm.P[k][tid];
     }
     if(CL)
+    {
         cluster_sync_all(); // no CTA leaves while its shared memory may be read
+        if(sm.failed)
+        {
+            // rank 0's pivots and info are written: identity pivots and INT_MIN over them
+            for(int c = j0 + tid; PIVOT && c < mn; c += NT)
+                M.piv[c] = c + 1;
+            if(tid == 0)
+                *M.info = INT_MIN;
+            // ... nor while a record is on its way to it.  Factoring warp 0 expected mysent[0]
+            // columns; of the last of them and the next, wait for the records that were sent.
+            if(warp == S && lane == 0 && lb.failed)
+            {
+                constexpr uint32_t RB = sizeof(PanelRec<T>);
+                const int nrec = nrank * SH::FW, last = sm.mysent[0] - 1;
+                int n0 = 0, n1 = 0;
+                for(int i = 0; i < nrec; ++i)
+                {
+                    n0 += sm.sent[i] > last;
+                    n1 += sm.sent[i] > last + 1;
+                }
+                if(n0 < nrec)
+                    mbar_complete(&sm.mbar[last & 1], (nrec - n0) * RB);
+                mbar_wait_cluster(&sm.mbar[last & 1], (lb.phase >> (last & 1)) & 1u,
+                                  CLUSTER_WAIT_LIMIT);
+                if(n1 > 0)
+                {
+                    mbar_expect(&sm.mbar[(last + 1) & 1], n1 * RB);
+                    mbar_wait_cluster(&sm.mbar[(last + 1) & 1],
+                                      (lb.phase >> ((last + 1) & 1)) & 1u, CLUSTER_WAIT_LIMIT);
+                }
+            }
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------- U12
@@ -824,7 +908,7 @@ __global__ void __launch_bounds__(TRSM_NT, sizeof(T) == 8 ? 3 : 5)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrsmSmem<T>& sm = *reinterpret_cast<TrsmSmem<T>*>(smem_raw);
     LuMember<T> M;
-    if(!lu_member(L, blockIdx.x / chunks, M))
+    if(!lu_member(L, blockIdx.x / chunks, M) || lu_gave_up(L, M))
         return;
     const int jb = min(NB, min(M.m, M.n) - j0);
     const int cfirst = j0 + jb + (blockIdx.x % chunks) * CW;
@@ -1204,7 +1288,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 3 : 4)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     GemmSmem<T>& sm = *reinterpret_cast<GemmSmem<T>*>(smem_raw);
     LuMember<T> M;
-    if(!lu_member(L, blockIdx.x / tiles, M))
+    if(!lu_member(L, blockIdx.x / tiles, M) || lu_gave_up(L, M))
         return;
     const int jb = min(NB, min(M.m, M.n) - j0);
     const int t = blockIdx.x % tiles;
@@ -1241,7 +1325,7 @@ __global__ void __launch_bounds__(LEFT_NT)
     int* s = perm + max_rows;
     __shared__ int piv[NB];
     LuMember<T> M;
-    if(!lu_member(L, blockIdx.x / (blocks * PARTS), M))
+    if(!lu_member(L, blockIdx.x / (blocks * PARTS), M) || lu_gave_up(L, M))
         return;
     const int t = blockIdx.x % (blocks * PARTS);
     const int c0 = (t / PARTS) * NB + (t % PARTS) * LEFT_COLS;

@@ -98,3 +98,86 @@ def test_blocked_sgetrf(handle, m, n):
     A = A[:, ::-1].copy()
     LU, ipiv, info, _ = gpu_getrf(handle, A)
     check_getrf(A, LU, ipiv, info)
+
+
+WAIT_CHILD = r'''
+import ctypes, os, sys
+import numpy as np
+import torch
+sys.path.insert(0, ROOT)
+import oracle
+import rocsolver_b200 as rs
+from tests.refcases import to_colmajor, uniform_general
+assert rs.LIB_PATH.endswith("_checked.so"), rs.LIB_PATH
+h = rs.Handle(torch.cuda.current_stream().cuda_stream)
+P = rs.ptr
+rec = (ctypes.c_int32 * 4)()
+GUARD, SENT, bc = 4096, -12345, 3
+for p, n in (("s", 300), ("s", 600), ("s", 1100), ("d", 600), ("d", 1100)):
+    dt, lda = np.float32 if p == "s" else np.float64, n + 3
+    A = (uniform_general(n, n, bc, seed=n) + 2 * n * np.eye(n)).astype(dt)[:, ::-1].copy()
+    flat = to_colmajor(A, lda).reshape(-1)
+    guard = np.full(GUARD, SENT, dt)
+    pad = np.ones((bc, n, lda), bool)
+    pad[:, :, :n] = False
+    for limit in ("0", "1", "3", None):
+        if limit is None:
+            del os.environ["ROCSOLVER_B200_CLUSTER_WAIT"]
+        else:
+            os.environ["ROCSOLVER_B200_CLUSTER_WAIT"] = limit
+        dA = torch.from_numpy(np.concatenate([guard, flat, guard])).cuda()
+        dP = torch.full((GUARD + bc * n + GUARD,), SENT, dtype=torch.int32, device="cuda")
+        dI = torch.full((GUARD + bc + GUARD,), SENT, dtype=torch.int32, device="cuda")
+        B = uniform_general(n, 2, bc, seed=5).astype(dt)
+        dB = torch.from_numpy(to_colmajor(B)).cuda()
+        B0 = dB.clone()
+        rs.check(rs.call(f"rocsolver_{p}gesv_strided_batched", h.value, n, 2, P(dA[GUARD:]), lda,
+                         lda * n, P(dP[GUARD:]), n, P(dB), n, 2 * n, P(dI[GUARD:]), bc), "gesv")
+        torch.cuda.synchronize()
+        rs.call("rocsolver_b200_bounds_check", ctypes.cast(rec, ctypes.c_void_p))
+        assert rec[0] == 0, (p, n, limit, list(rec))
+        a, ip, info = dA.cpu().numpy(), dP.cpu().numpy(), dI.cpu().numpy()
+        for x in (a, ip, info):
+            assert (x[:GUARD] == SENT).all() and (x[-GUARD:] == SENT).all(), (p, n, limit)
+        a, ip, info = a[GUARD:-GUARD], ip[GUARD:-GUARD].reshape(bc, n), info[GUARD:-GUARD]
+        assert np.isnan(a.reshape(bc, n, lda)[pad]).all()  # to_colmajor pads with NaN
+        assert (ip >= np.arange(1, n + 1)).all() and (ip <= n).all(), (p, n, limit)
+        gave_up = info == np.iinfo(np.int32).min
+        print(p, n, limit, "members given up", int(gave_up.sum()), flush=True)
+        assert ((info == 0) | gave_up).all(), (p, n, limit, info)
+        if limit == "0":
+            assert gave_up.all()
+        if limit is None:
+            assert not gave_up.any()
+        oA, oP, oI = to_colmajor(A).copy(), np.zeros(bc * n, np.int32), np.zeros(bc, np.int32)
+        oracle.getrf(n, n, oA, n, n * n, oP, n, oI, bc, nthreads=oracle.nthreads_default())
+        for b in range(bc):
+            if gave_up[b]:
+                assert torch.equal(dB.view(bc, -1)[b], B0.view(bc, -1)[b])
+            else:
+                assert (ip[b] == oP.reshape(bc, n)[b]).all()
+                x = dB.view(bc, 2, n)[b].cpu().numpy().astype(np.float64).T
+                r = np.abs(A[b].astype(np.float64) @ x - B[b]).max()
+                assert r <= n * np.finfo(dt).eps * (np.abs(A[b]).sum(1).max() * np.abs(x).max())
+h.close()
+print("waits done")
+'''
+
+
+def test_cluster_wait_that_runs_out():
+    """A wait between the CTAs of a panel's cluster that runs out ends in info = INT_MIN, pivots
+    in range, the right-hand sides of gesv as they were, and nothing written outside the member
+    (the checked build: limits of 0, 1 and 3 polls, so that the CTAs give up at different
+    columns); the call after it, with the usual limit, is right."""
+    import os
+    import subprocess
+    import sys
+    if not os.path.exists(rs.CHECKED_LIB_PATH):
+        pytest.skip("bounds-checked library not built (python -m rocsolver_b200.build --checked)")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, ROCSOLVER_B200_LIB=rs.CHECKED_LIB_PATH,
+               ROCSOLVER_B200_CLUSTER_WAIT="0")
+    r = subprocess.run([sys.executable, "-c", "ROOT = " + repr(root) + "\n" + WAIT_CHILD], env=env,
+                       capture_output=True, text=True, timeout=600, cwd=root)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+    assert "waits done" in r.stdout
