@@ -1,4 +1,5 @@
-"""Autotuner for the CTA LU kernels and the persistent variable-size kernel.
+"""Autotuner: the CTA LU kernels against the library's built-in choice, and the persistent
+variable-size kernel's configurations.
 
     python -m rocsolver_b200.tune [--out PATH] [--quick] [--classes 64,128,256,...]
 
@@ -7,7 +8,9 @@ Replaces the reference's hand-set compile-time tables (library/src/include/ideal
 For every size class and precision it times each compiled configuration that can take
 the class's largest size -- (threads, rows per thread, panel width), trailing-update
 column chunk, and whether the panel's row interchanges are folded into the trailing
-update -- on seeded uniform[-1, 1] batches, and keeps the fastest.  For the variable-size
+update -- on seeded uniform[-1, 1] batches, and keeps the fastest, or the built-in choice (for
+most sizes the blocked LU) where no configuration beats it: the class then gets a row of zeros,
+which names no configuration and keeps the next class's row from applying to it.  For the variable-size
 kernel it also tunes the number of resident CTAs per SM, on batches with n uniform in
 [8, n_max] and nrhs uniform in [1, 16].  Precision t is the FP32 LU with split-TF32
 trailing updates (rocsolver_sgetrf_tf32_strided_batched, the factorisation of dsgesv); its
@@ -16,10 +19,11 @@ candidates include the tcgen05 trailing update (fold = 2) for the variants compi
 The table (format in include/rocsolver.h, rocsolver_b200_tuning_set) is written to
 rocsolver_b200/tuning_b200.txt by default, where the library reads it when the first
 handle is created.  Every candidate's pivots are compared with the built-in
-configuration's on the same input; results do not depend on the table, only speed does.
+choice's on the same input; apart from rounding, results do not depend on the table.
 """
 import argparse
 import datetime
+import math
 import os
 import statistics
 
@@ -101,7 +105,7 @@ def tune_getrf(prec, n, bc, reps, quick, log):
         rs.set_tuning_table("")
         t_builtin = _time(call, reset, reps)
         piv_ref = ipiv.clone()
-        best = None
+        best = (math.inf, None)
         for cand in _lu_candidates(n, quick, prec):
             nt, r, jb, cw, fold = cand
             rs.set_tuning_table(f"getrf {prec} {n} {nt} {r} {jb} {cw} {fold}\n")
@@ -110,7 +114,7 @@ def tune_getrf(prec, n, bc, reps, quick, log):
             bad = int((info != 0).sum()) + int((~torch.isfinite(A)).sum())
             log(f"  getrf {prec} n={n} bc={bc} {cand}: {t:.3f} ms  pivot mismatches {mism}"
                 f"  bad {bad}")
-            if bad == 0 and (best is None or t < best[0]):
+            if bad == 0 and t < best[0]:
                 best = (t, cand)
         log(f"getrf {prec} n={n}: built-in {t_builtin:.3f} ms, best {best[1]} {best[0]:.3f} ms")
         return best[1], best[0], t_builtin
@@ -158,7 +162,7 @@ def tune_vbatched(prec, nmax, bc, reps, quick, log):
         rs.set_tuning_table("")
         t_builtin = _time(call, reset, reps)
         piv_ref = ipiv.clone()
-        best = None
+        best = (math.inf, None)
         for nt, r, jb in VB_VARIANTS:
             if nt * r < nmax or nt * r >= 4 * nmax:
                 continue
@@ -173,13 +177,22 @@ def tune_vbatched(prec, nmax, bc, reps, quick, log):
                         bad = int((info != 0).sum())
                         log(f"  vbatched {prec} n_max={nmax} bc={bc} {cand}: {t:.3f} ms  "
                             f"pivot mismatches {mism}  bad {bad}")
-                        if bad == 0 and (best is None or t < best[0]):
+                        if bad == 0 and t < best[0]:
                             best = (t, cand)
         log(f"vbatched {prec} n_max={nmax}: built-in {t_builtin:.3f} ms, best {best[1]} "
             f"{best[0]:.3f} ms")
         return best[1], best[0], t_builtin
     finally:
         h.close()
+
+
+def _row(kind, prec, n, cand, t, t_builtin, batch, nvals):
+    """The class's table row: the configuration where it beats the built-in choice, else zeros."""
+    if cand is None or t >= t_builtin:
+        return (f"{kind} {prec} {n}" + " 0" * nvals
+                + f"    # built-in: {t_builtin:.3f} ms, best other {t:.3f} ms, batch {batch}")
+    return (f"{kind} {prec} {n} " + " ".join(map(str, cand))
+            + f"    # {t:.3f} / {t_builtin:.3f} ms, batch {batch}")
 
 
 def main():
@@ -214,13 +227,11 @@ def main():
             for n in [int(x) for x in a.classes.split(",") if x]:
                 cand, t, tb = tune_getrf(prec, n, GETRF_CLASSES.get(n, 256), a.reps, a.quick,
                                          log)
-                lines.append(f"getrf {prec} {n} " + " ".join(map(str, cand))
-                             + f"    # {t:.3f} / {tb:.3f} ms, batch {GETRF_CLASSES.get(n, 256)}")
+                lines.append(_row("getrf", prec, n, cand, t, tb, GETRF_CLASSES.get(n, 256), 5))
             for n in [int(x) for x in a.vb_classes.split(",") if x and prec != "t"]:
                 cand, t, tb = tune_vbatched(prec, n, VB_CLASSES.get(n, 1024), a.reps, a.quick,
                                             log)
-                lines.append(f"vbatched {prec} {n} " + " ".join(map(str, cand))
-                             + f"    # {t:.3f} / {tb:.3f} ms, batch {VB_CLASSES.get(n, 1024)}")
+                lines.append(_row("vbatched", prec, n, cand, t, tb, VB_CLASSES.get(n, 1024), 6))
     finally:
         rs.set_tuning_table(old)
     if a.merge and os.path.exists(a.out):

@@ -70,3 +70,42 @@ def test_get_truncates_to_buffer():
         assert buf.value == b"getrf d"
     finally:
         _restore(old)
+
+
+def test_tuner_keeps_the_built_in_choice_where_it_is_faster(tmp_path, monkeypatch):
+    """A class whose best configuration is slower than the built-in choice gets a row of zeros
+    (no configuration), also between classes that have one, and the library takes the file."""
+    import sys
+
+    import torch
+
+    from rocsolver_b200 import tune
+    times = {("d", 64): (1.6, 1.1), ("d", 128): (2.5, 3.0), ("s", 64): (1.0, 1.0),
+             ("s", 128): (float("inf"), 2.0)}
+
+    def fake_getrf(prec, n, bc, reps, quick, log):
+        t, tb = times[prec, n]
+        return (None if t == float("inf") else (256, 1, 32, 64, 1)), t, tb
+
+    def fake_vbatched(prec, n, bc, reps, quick, log):
+        return (256, 2, 32, 128, 0, 0), (5.0 if prec == "d" else 3.0), 4.0
+
+    monkeypatch.setattr(tune, "tune_getrf", fake_getrf)
+    monkeypatch.setattr(tune, "tune_vbatched", fake_vbatched)
+    monkeypatch.setattr(torch.cuda, "get_device_name", lambda *a: "none")
+    out = tmp_path / "table.txt"
+    monkeypatch.setattr(sys, "argv", ["tune", "--out", str(out), "--classes", "64,128",
+                                      "--vb-classes", "512", "--precisions", "d,s"])
+    old = rs.tuning_table()
+    tune.main()
+    assert rs.tuning_table() == old
+    try:
+        assert rs.lib().rocsolver_b200_tuning_load(str(out).encode()) == SUCCESS
+        assert rs.tuning_table().splitlines() == ["getrf d 64 0 0 0 0 0",
+                                                  "getrf d 128 256 1 32 64 1",
+                                                  "getrf s 64 0 0 0 0 0",
+                                                  "getrf s 128 0 0 0 0 0",
+                                                  "vbatched d 512 0 0 0 0 0 0",
+                                                  "vbatched s 512 256 2 32 128 0 0"]
+    finally:
+        _restore(old)
