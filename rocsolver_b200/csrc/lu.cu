@@ -63,6 +63,93 @@ static void run_getrf_warp(cudaStream_t s, int m, int n, Batch<T> A, int lda, in
                                                                        info, bc, g);
 }
 
+// Without a table entry: whether the one-launch CTA kernels (one CTA holds a member from first
+// to last panel) take a call, or the blocked LU in separate launches.
+//
+// FP64 up to 512 rows: the CTA kernels, always.  These factors feed inverses and adjoints of
+// matrices whose condition nothing bounds (uniform + 4 I, 16384 members of n = 64, hold one of
+// 1e7 now and then), where another order of rounding shows: with the blocked LU such outputs
+// moved by 1e-9 to 4e-9 (relative, 2-norm) in one of ten to one of four batches of n = 64 ..
+// 256, beyond the 5e-10 that they are held to, at the same error against 64-bit results.  The
+// blocked LU is no clear gain there either (getrf alone, ms, blocked / CTA): n = 64 x 16384
+// 1.06 / 1.63, n = 65 x 16384 3.08 / 2.64, n = 128 x 8178 2.52 / 3.04, n = 129 x 8052 5.65 /
+// 4.52, n = 200 x 3350 4.80 / 4.06, n = 256 x 2044 3.52 / 3.79, n = 512 x 592 6.95 / 7.12.
+//
+// Else the faster one.  The blocked LU pays for a whole 64-column panel, and for rows up to 64,
+// 128, 256 or a cluster of 2, 4 or 8 CTAs of 256, whatever part of them a member fills; a
+// cluster's CTA has an SM to itself, so clusters of 2 take 74 members at a time where the CTA
+// kernels take 148; and the CTA kernels lose a part of their last wave.  Time of the CTA kernel
+// over that of the blocked LU, at batches from 1 to 134e6 / n^2:
+//   rows       FP32          split TF32
+//   33-64      1.4-1.7       1.5-2.7
+//   65-96      0.82-1.18     0.83-1.17
+//   97-128     1.08-1.57     1.08-1.60
+//   129-160    0.71-1.15     0.68-1.13
+//   161-192    0.99-1.57     to 296 members 1.16-1.53, then 0.91-1.35
+//   193-224    to 296 members 1.02-1.48, then 0.82-1.12;  to 222 1.04-1.40, then 0.73-1.05
+//   225-256    1.08-1.91     to 296 members 1.14-1.83, then n < 250 0.90-1.24, 256 1.10-1.35
+//   257-512    to 74 members 0.99-2.3 (TF32 below 284 rows 0.90-1.02), 75-148 0.73-1.16,
+//              then 0.90-1.57 (TF32 0.77-1.33); at least 1.04 for 284 to 320 rows and, FP32,
+//              above 480 rows and at multiples of 64
+//   513-2048   1.2-57        0.96-23  (FP64 0.95-38)
+// Panels with few columns (2 n <= m, more than 256 rows) have nothing to update beside the
+// clusters: 300 x 64 0.42-0.84, 500 x 250 to 74 members 1.2, then 0.7; 1000 x 64 to 37 members
+// 1.1 and 2.2, then 0.5; 2000 x 64 to 74 members 1.2 and 3.0, then 0.6 (FP64 0.83 at 74).
+template <typename T>
+static bool cta_lu_pays(int m, int n, int bc, bool tc)
+{
+    if(sizeof(T) == 8 && m <= 512)
+        return true;
+    if(m <= 64 || n >= 2 * m)
+        return false;
+    if(m > 256 && 2 * n <= m)
+    {
+        const int cluster = m <= 512 ? 2 : (m <= 1024 ? 4 : 8);
+        return m <= 400 || (int64_t)bc * cluster * 700 > (int64_t)132 * std::max(m, 700);
+    }
+    if(m <= 96)
+        return true;
+    if(m <= 128)
+        return false;
+    if(m <= 160)
+        return true;
+    if(m <= 192)
+        return tc && bc > 296;
+    if(m <= 224)
+        return bc > (tc ? 222 : 296);
+    if(m <= 256)
+        return tc && m < 250 && bc > 296;
+    if(m <= 512)
+    {
+        if(bc <= 74)
+            return tc && m < 284;
+        if(bc <= 148)
+            return true;
+        const bool full = m >= 284 && m <= 320;
+        return !(full || (!tc && (m > 480 || m % 64 == 0)));
+    }
+    return false;
+}
+
+// the CTA variant of a size (measured by rocsolver_b200/tune.py at the largest rows of each)
+template <typename T>
+static LuCfg cta_lu_builtin(int m, bool tc)
+{
+    if(sizeof(T) == 8)
+        return m <= 64     ? LuCfg{128, 1, 32, 32, 1}
+               : m <= 128  ? LuCfg{128, 1, 32, 64, 1}
+               : m <= 256  ? LuCfg{256, 1, 32, 64, 1}
+               : m <= 512  ? LuCfg{256, 2, 32, 128, 1}
+               : m <= 1024 ? LuCfg{256, 4, 16, 128, 1}
+                           : LuCfg{256, 8, 8, 96, 1};
+    return m <= 128    ? LuCfg{128, 2, 32, 128, 1}
+           : m <= 256  ? LuCfg{128, 2, 32, 64, 1}
+           : m <= 512  ? LuCfg{256, 2, 32, 128, 1}
+           : m <= 1024 ? LuCfg{256, 4, 16, 128, 1}
+           : tc        ? LuCfg{256, 8, 8, 128, 3}
+                       : LuCfg{256, 8, 8, 32, 1};
+}
+
 template <typename T, bool PIVOT, bool TC>
 static rocblas_status getrf_dispatch(cudaStream_t s, int m, int n, Batch<T> A, int lda,
                                      int* ipiv, int64_t sP, int* info, int bc, Gate g)
@@ -87,27 +174,14 @@ static rocblas_status getrf_dispatch(cudaStream_t s, int m, int n, Batch<T> A, i
         if(ran)
             return st;
     }
-    // Without an entry, FP64 up to 512 rows: the one-launch CTA kernels.  The factors feed
-    // inverses and adjoints of matrices whose condition nothing bounds (uniform + 4 I, 16384
-    // members of n = 64, hold one of 1e7 now and then), where another order of rounding shows:
-    // with the blocked LU these outputs moved by 1e-9 to 4e-9 (relative, 2-norm) in one of ten
-    // to one of four batches of n = 64 .. 256, beyond the 5e-10 that such solves are held to,
-    // at the same error against 64-bit results.  The blocked LU is no clear gain there either
-    // (getrf alone, ms, blocked / CTA): n = 64 x 16384 1.06 / 1.63, n = 65 x 16384 3.08 / 2.64,
-    // n = 128 x 8178 2.52 / 3.04, n = 129 x 8052 5.65 / 4.52, n = 200 x 3350 4.80 / 4.06,
-    // n = 256 x 2044 3.52 / 3.79, n = 512 x 592 6.95 / 7.12.
-    if(sizeof(T) == 8 && m <= 512)
+    if(cta_lu_pays<T>(m, n, bc, TC))
     {
-        const LuCfg d = m <= 64    ? LuCfg{64, 1, 32, 0, 0}
-                        : m <= 128 ? LuCfg{128, 1, 32, 0, 0}
-                        : m <= 256 ? LuCfg{256, 1, 32, 0, 0}
-                                   : LuCfg{256, 2, 16, 0, 0};
         bool ran = false;
-        return run_getrf_tuned<T, PIVOT, TC>(d, s, m, n, A, lda, ipiv, sP, info, bc, g, &ran);
+        const rocblas_status st = run_getrf_tuned<T, PIVOT, TC>(
+            cta_lu_builtin<T>(m, TC), s, m, n, A, lda, ipiv, sP, info, bc, g, &ran);
+        if(ran)
+            return st;
     }
-    // The rest: the blocked LU in separate launches.  Measured against the CTA kernels with
-    // their tuned entries (getrf alone, ms, blocked / CTA): FP64 n = 2048 x 16 10.3 / 161; FP32
-    // n = 501 x 200 2.09 / 2.93; split TF32 n = 256 x 2048 2.00 / 2.23.
     LuBatch<T> L{};
     L.A = A;
     L.m = m;

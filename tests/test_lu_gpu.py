@@ -139,6 +139,44 @@ def test_dgetrf_rounds_as_the_cta_kernel(handle, n):
     np.testing.assert_array_equal(LU, LU2)
 
 
+# (rows, columns, members, whether one CTA per member takes them): both sides of each line of
+# the built-in choice
+ROUTES = [(64, 64, 3, False), (65, 65, 3, True), (96, 96, 3, True), (97, 97, 3, False),
+          (128, 128, 3, False), (129, 129, 3, True), (160, 160, 3, True), (161, 161, 3, False),
+          (193, 193, 296, False), (193, 193, 297, True), (225, 225, 297, False),
+          (257, 257, 74, False), (257, 257, 75, True), (257, 257, 149, True),
+          (284, 284, 149, False), (320, 320, 148, True), (321, 321, 149, True),
+          (384, 384, 149, False), (481, 481, 149, False), (513, 513, 3, False),
+          (65, 130, 3, False), (400, 200, 3, True), (402, 201, 3, False), (402, 201, 67, True),
+          (900, 64, 42, False), (900, 64, 43, True)]
+
+
+@pytest.mark.parametrize("m,n,bc,cta", ROUTES)
+def test_sgetrf_either_side_of_the_built_in_choice(handle, m, n, bc, cta):
+    """Each route gives the oracle's pivots and factors; that the route is the expected one shows
+    in the bits, which are those of the CTA kernel on one side only."""
+    rng = np.random.default_rng(m * 1000 + bc)
+    A = rng.uniform(-1, 1, (bc, m, n)).astype(np.float32)
+    for b in range(bc):  # one large entry per column, in rows drawn at random
+        A[b, rng.permutation(max(m, n))[:n] % m, np.arange(n)] += 6 + 0.2 * n
+    LU, ipiv, info, _ = gpu_getrf(handle, A)
+    if n <= m:
+        some = slice(0, min(bc, 4))
+        mn = min(m, n)
+        check_getrf(A[some], LU[some], ipiv[:mn * min(bc, 4)], info[some])
+    old = rs.tuning_table()
+    try:
+        row = ("128 2 32 64 1" if m <= 256 else "256 2 32 128 1" if m <= 512
+               else "256 4 16 128 1")
+        assert rs.set_tuning_table(f"getrf s {m} {row}\n") == rs.SUCCESS
+        forced, fpiv, finfo, _ = gpu_getrf(handle, A)
+    finally:
+        assert rs.set_tuning_table(old) == rs.SUCCESS
+    np.testing.assert_array_equal(ipiv, fpiv)
+    np.testing.assert_array_equal(info, finfo)
+    assert np.array_equal(LU, forced) == cta
+
+
 @pytest.mark.parametrize("n", [16, 33, 64, 100, 128, 200, 256, 300, 512, 1024])
 def test_sgetrf_tf32(handle, n):
     """rocsolver_sgetrf_tf32_strided_batched (split-TF32 tensor-core trailing updates, the
