@@ -30,25 +30,32 @@ namespace rsb {
 // groups of 8.  Each row stores its column-c entry as it is finalised.
 // A non-positive or NaN pivot at step c: columns < c are final, A(c, c) keeps the updated
 // value, the rest of the matrix is untouched and info = c + 1 (LAPACK dpotf2).
-// UPPER: the triangle is staged in shared memory on the way in and out, along its stored
-// columns.  j0: the block of n columns at (j0, j0) of a larger member (blocked potrf); members
-// whose info is already set are left alone.
-template <typename T, int N, bool UPPER>
+// UPPER: M(r, c) = A(c, r).  BLOCK: the n columns at (j0, j0) of a larger member (blocked
+// potrf); members whose info is already set are left alone, and the upper triangle is staged in
+// shared memory on the way in and out, along its stored columns.  Whole members of the upper
+// case are not staged: the extra pass costs a small batch more than the strided accesses (FP64
+// n = 32 x 16 14.2 against 10.1 us staged / direct, n = 48 x 148 21.2 / 17.0), and a large one
+// at most orders (n = 24 x 20000 122 / 101 us, n = 48 x 20000 565 / 477, n = 64 x 20000 750 /
+// 752; gains were FP32 n = 64 x 20000 449 / 508 and n = 32 x 20000 92 / 123).
+template <typename T, int N, bool UPPER, bool BLOCK>
 __global__ void __launch_bounds__(N, N <= 32 ? 16 : 6)
     potrf_reg_kernel(int n, Batch<T> A, int lda, int* info, int j0)
 {
-    __shared__ T tri[UPPER ? N : 1][N + 1]; // [row][column]
+    constexpr bool STAGE = UPPER && BLOCK;
+    __shared__ T tri[STAGE ? N : 1][N + 1]; // [row][column]
     // published column (slot r - c); rows of N + 4 elements keep both buffers 16-byte
     // aligned for the vector reads in FP32 and FP64
     __shared__ __align__(16) T scol[2][N + 4];
     __shared__ T sdiag[2][2];                  // sqrt(pivot), 1/sqrt(pivot)
     const int r = threadIdx.x;
     const int64_t b = blockIdx.x;
-    if(j0 > 0 && info[b] != 0)
+    if(BLOCK && j0 > 0 && info[b] != 0)
         return;
-    T* a = A.at(b) + ix(j0, j0, lda);
-    auto at = [&](int i, int j) -> T& { return UPPER ? tri[i][j] : a[ix(i, j, lda)]; };
-    if(UPPER)
+    T* a = A.at(b) + (BLOCK ? ix(j0, j0, lda) : 0);
+    auto at = [&](int i, int j) -> T& {
+        return STAGE ? tri[i][j] : (UPPER ? a[ix(j, i, lda)] : a[ix(i, j, lda)]);
+    };
+    if(STAGE)
     {
 #pragma unroll 8
         for(int i = 0; i < n; ++i)
@@ -126,15 +133,15 @@ __global__ void __launch_bounds__(N, N <= 32 ? 16 : 6)
             }
         }
     }
-    if(UPPER)
+    if(STAGE)
     {
         __syncthreads();
         for(int i = 0; i < n; ++i)
             if(r <= i)
                 a[ix(r, i, lda)] = tri[i][r];
     }
-    if(r == 0 && (j0 == 0 || inf != 0))
-        info[b] = inf != 0 ? j0 + inf : 0;
+    if(r == 0 && (!BLOCK || j0 == 0 || inf != 0))
+        info[b] = inf != 0 && BLOCK ? j0 + inf : inf;
 }
 
 } // namespace rsb

@@ -318,15 +318,15 @@ rocblas_status launch_gesv(cudaStream_t s, int n, int nrhs, Batch<T> A, int lda,
 }
 
 // ------------------------------------------------------------------------------ potrf
-template <typename T, int N>
+template <typename T, int N, bool BLOCK>
 static rocblas_status run_potrf_reg(cudaStream_t s, int upper, int n, Batch<T> A, int lda,
                                     int* info, int bc, int j0 = 0)
 {
     RSB_LOG_KERNEL("potrf_reg_kernel");
     if(upper)
-        potrf_reg_kernel<T, N, true><<<bc, N, 0, s>>>(n, A, lda, info, j0);
+        potrf_reg_kernel<T, N, true, BLOCK><<<bc, N, 0, s>>>(n, A, lda, info, j0);
     else
-        potrf_reg_kernel<T, N, false><<<bc, N, 0, s>>>(n, A, lda, info, j0);
+        potrf_reg_kernel<T, N, false, BLOCK><<<bc, N, 0, s>>>(n, A, lda, info, j0);
     return launch_status();
 }
 
@@ -341,9 +341,9 @@ static rocblas_status run_potrf_blk(cudaStream_t s, int n, Batch<T> A, int lda, 
     for(int j0 = 0; j0 < n; j0 += NB)
     {
         const int jb = std::min(NB, n - j0), below = n - j0 - jb;
-        const rocblas_status st = jb <= 32
-                                      ? run_potrf_reg<T, 32>(s, UPPER, jb, A, lda, info, bc, j0)
-                                      : run_potrf_reg<T, 64>(s, UPPER, jb, A, lda, info, bc, j0);
+        const rocblas_status st =
+            jb <= 32 ? run_potrf_reg<T, 32, true>(s, UPPER, jb, A, lda, info, bc, j0)
+                     : run_potrf_reg<T, 64, true>(s, UPPER, jb, A, lda, info, bc, j0);
         if(st != rocblas_status_success || below <= 0)
             return st;
         const int chunks = (below + CHOL_CW - 1) / CHOL_CW, t = (below + 63) / 64;
@@ -372,9 +372,9 @@ rocblas_status launch_potrf(cudaStream_t s, int upper, int n, Batch<T> A, int ld
                             int bc)
 {
     if(n <= 32)
-        return run_potrf_reg<T, 32>(s, upper, n, A, lda, info, bc);
+        return run_potrf_reg<T, 32, false>(s, upper, n, A, lda, info, bc);
     if(n <= 64)
-        return run_potrf_reg<T, 64>(s, upper, n, A, lda, info, bc);
+        return run_potrf_reg<T, 64, false>(s, upper, n, A, lda, info, bc);
     if(n > MAX_CTA_ROWS)
         return rocblas_status_not_implemented;
     return upper ? run_potrf_blk<T, true>(s, n, A, lda, info, bc)
