@@ -41,8 +41,7 @@ rocblas_status panel(cudaStream_t s, const LuBatch<T>& L, int j0, int lo, int hi
     const size_t smem = sizeof(PanelSmem<T, BLK_NB, S>);
     if(!set_smem(k, smem))
         return rocblas_status_internal_error;
-    // (traces keep the name of the CTA factorisation)
-    RSB_LOG_KERNEL("getrf_cta_kernel");
+    RSB_LOG_KERNEL("getrf_panel_kernel");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((int64_t)bc * cluster));
     cfg.blockDim = dim3(PanelShape<T, S>::NT);

@@ -132,6 +132,34 @@ def test_trace_kernels_and_profile_gpu(tmp_path, monkeypatch):
     assert "    getrf_cta_kernel: Calls: 2, Total Time:" in text
 
 
+@pytest.mark.gpu
+def test_profile_names_the_kernels_of_the_blocked_lu(tmp_path, monkeypatch):
+    """n = 520 in FP64 takes the blocked LU: nine panels, eight interchange and update launches,
+    one for L's rows, and no launch of the CTA kernel."""
+    import torch
+    path = tmp_path / "log.txt"
+    monkeypatch.setenv("ROCSOLVER_LOG_PATH", str(path))
+    monkeypatch.setenv("ROCSOLVER_LAYER", str(4 | 0x10))
+    monkeypatch.setenv("ROCSOLVER_LEVELS", "3")
+    assert rs.call("rocsolver_log_begin") == rs.SUCCESS
+    h = rs.Handle(torch.cuda.current_stream().cuda_stream)
+    try:
+        n, bc = 520, 2
+        A = torch.rand(bc, n, n, dtype=torch.float64, device="cuda")
+        P = torch.zeros(bc * n, dtype=torch.int32, device="cuda")
+        I = torch.zeros(bc, dtype=torch.int32, device="cuda")
+        rs.check(rs.call("rocsolver_dgetrf_strided_batched", h.value, n, n, rs.ptr(A), n, n * n,
+                         rs.ptr(P), n, rs.ptr(I), bc), "getrf")
+        torch.cuda.synchronize()
+    finally:
+        h.close()
+    assert rs.call("rocsolver_log_end") == rs.SUCCESS
+    text = path.read_text()
+    for name, calls in (("panel", 9), ("swap_trsm", 8), ("gemm", 8), ("left", 1)):
+        assert f"    getrf_{name}_kernel: Calls: {calls}, Total Time:" in text
+    assert "getrf_cta_kernel" not in text
+
+
 def test_complex_entry_points_log_their_precision(session):
     """The c / z entry points log with -r c / -r z, as the reference's do
     (rocsolver_logger.hpp get_precision for rocblas_float_complex / rocblas_double_complex),
