@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(CHOL_NT, sizeof(T) == 8 ? 3 : 5)
     T* a = A.at(b);
     const int r0 = j0 + NB + (blockIdx.x % chunks) * CHOL_CW;
     const int nr = min(CHOL_CW, n - r0);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5;
     auto at = [&](int r, int c) -> T& {
         return UPPER ? RSB_AT(a, c, r, lda, n, n) : RSB_AT(a, r, c, lda, n, n);
     };
@@ -69,44 +69,7 @@ __global__ void __launch_bounds__(CHOL_NT, sizeof(T) == 8 ? 3 : 5)
         if constexpr(sizeof(T) == 8)
         {
             if(ib > 0 && warp * 16 < nr)
-            {
-                const int g = lane >> 2, q = lane & 3;
-                double* x = &sm.X[warp * 16][0];
-                double acc[2][2][2];
-#pragma unroll
-                for(int i = 0; i < 2; ++i)
-#pragma unroll
-                    for(int j = 0; j < 2; ++j)
-#pragma unroll
-                        for(int e = 0; e < 2; ++e)
-                            acc[i][j][e] = x[(8 * j + 2 * q + e) * (NB + 1) + ib + 8 * i + g];
-#pragma unroll 4
-                for(int k = 0; k < ib; k += 4)
-                {
-                    double l[2], y[2];
-#pragma unroll
-                    for(int i = 0; i < 2; ++i)
-                    {
-                        l[i] = -sm.L[k + q][ib + 8 * i + g];
-                        y[i] = x[(8 * i + g) * (NB + 1) + k + q];
-                    }
-#pragma unroll
-                    for(int i = 0; i < 2; ++i)
-#pragma unroll
-                        for(int j = 0; j < 2; ++j)
-                            asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
-                                         "{%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                                         : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
-                                         : "d"(l[i]), "d"(y[j]));
-                }
-#pragma unroll
-                for(int i = 0; i < 2; ++i)
-#pragma unroll
-                    for(int j = 0; j < 2; ++j)
-#pragma unroll
-                        for(int e = 0; e < 2; ++e)
-                            x[(8 * j + 2 * q + e) * (NB + 1) + ib + 8 * i + g] = acc[i][j][e];
-            }
+                trsm_tile(sm.L, &sm.X[warp * 16][0], ib);
             __syncthreads();
         }
         if(tid < nr)

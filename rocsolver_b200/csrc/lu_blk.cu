@@ -34,12 +34,11 @@ int cluster_wait_limit()
 }
 
 template <typename T, int S, bool PIVOT, bool CL>
-rocblas_status panel(cudaStream_t s, const LuBatch<T>& L, int j0, int lo, int hi, int bc,
-                     int cluster)
+rocblas_status panel(cudaStream_t s, const LuBatch<T>& L, int j0, int bc, int cluster, bool first)
 {
     auto k = lu_panel_kernel<T, BLK_NB, S, PIVOT, CL>;
-    const size_t smem = sizeof(PanelSmem<T, BLK_NB, S>);
-    if(!set_smem(k, smem))
+    const size_t smem = sizeof(PanelSmem<T, BLK_NB, S, CL>);
+    if(first && !set_smem(k, smem))
         return rocblas_status_internal_error;
     RSB_LOG_KERNEL("getrf_panel_kernel");
     cudaLaunchConfig_t cfg = {};
@@ -53,24 +52,30 @@ rocblas_status panel(cudaStream_t s, const LuBatch<T>& L, int j0, int lo, int hi
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = CL ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k, L, j0, lo, hi, cluster_wait_limit()) == cudaSuccess
+    return cudaLaunchKernelEx(&cfg, k, L, j0, cluster_wait_limit()) == cudaSuccess
                ? launched()
                : rocblas_status_internal_error;
 }
 
-// the panel at j0 of members with lo < rows <= hi: the smallest CTA that holds hi rows, or a
-// cluster of CTAs of 256 rows
-template <typename T, bool PIVOT>
-rocblas_status panel_rows(cudaStream_t s, const LuBatch<T>& L, int j0, int lo, int hi, int bc)
+// CTAs of 64, 128 or 256 rows (1, 2, 3) or clusters of CTAs of 256 (4)
+int panel_class(int rows)
 {
-    if(hi <= 64)
-        return panel<T, 2, PIVOT, false>(s, L, j0, lo, hi, bc, 1);
-    if(hi <= 128)
-        return panel<T, 4, PIVOT, false>(s, L, j0, lo, hi, bc, 1);
-    if(hi <= 256)
-        return panel<T, 8, PIVOT, false>(s, L, j0, lo, hi, bc, 1);
-    const int cluster = hi <= 512 ? 2 : (hi <= 1024 ? 4 : 8);
-    return panel<T, 8, PIVOT, true>(s, L, j0, lo, hi, bc, cluster);
+    return rows <= 64 ? 1 : rows <= 128 ? 2 : rows <= 256 ? 3 : 4;
+}
+
+// the panel at j0: the smallest CTA that holds the rows, or a cluster of CTAs of 256 rows;
+// first: this class's kernel has not been launched in this call
+template <typename T, bool PIVOT>
+rocblas_status panel_rows(cudaStream_t s, const LuBatch<T>& L, int j0, int rows, int bc,
+                          bool first)
+{
+    switch(panel_class(rows))
+    {
+    case 1: return panel<T, 2, PIVOT, false>(s, L, j0, bc, 1, first);
+    case 2: return panel<T, 4, PIVOT, false>(s, L, j0, bc, 1, first);
+    case 3: return panel<T, 8, PIVOT, false>(s, L, j0, bc, 1, first);
+    }
+    return panel<T, 8, PIVOT, true>(s, L, j0, bc, rows <= 512 ? 2 : (rows <= 1024 ? 4 : 8), first);
 }
 
 template <typename T, bool PIVOT, bool TC>
@@ -78,26 +83,22 @@ rocblas_status lu_blk(cudaStream_t s, const LuBatch<T>& L, int m, int n, int bc)
 {
     constexpr int NB = BLK_NB;
     const int mn = std::min(m, n);
-    const bool var = L.v.n != nullptr;
     rocblas_status st = rocblas_status_success;
+    int cls = 0;
     for(int j0 = 0; j0 < mn; j0 += NB)
     {
-        const int mp = m - j0, jb = std::min(NB, mn - j0);
-        // members of a variable-size batch differ in their rows: one launch per class
-        static const int edge[] = {0, 64, 128, 256, 512, 1024, 2048};
-        for(int e = 1; e < 7 && st == rocblas_status_success; ++e)
-            if(var ? mp > edge[e - 1] : mp > edge[e - 1] && mp <= edge[e])
-                st = panel_rows<T, PIVOT>(s, L, j0, edge[e - 1], std::min(edge[e], mp), bc);
+        const int rows = m - j0, jb = std::min(NB, mn - j0);
+        const bool first = panel_class(rows) != cls;
+        cls = panel_class(rows);
+        st = panel_rows<T, PIVOT>(s, L, j0, rows, bc, first);
         if(st != rocblas_status_success)
             return st;
-        // variable sizes: a smaller member may have a narrower last panel, so its trailing
-        // columns (none: square members) need no launch of their own
         const int right = n - j0 - jb, below = m - j0 - jb;
         if(right <= 0)
             break;
         {
             auto k = lu_swap_trsm_kernel<T, PIVOT>;
-            if(!set_smem(k, sizeof(TrsmSmem<T>)))
+            if(j0 == 0 && !set_smem(k, sizeof(TrsmSmem<T>)))
                 return rocblas_status_internal_error;
             const int chunks = (right + TRSM_CW - 1) / TRSM_CW;
             RSB_LOG_KERNEL("getrf_swap_trsm_kernel");
@@ -108,7 +109,7 @@ rocblas_status lu_blk(cudaStream_t s, const LuBatch<T>& L, int m, int n, int bc)
         if(below > 0)
         {
             auto k = lu_gemm_kernel<T, TC>;
-            if(!set_smem(k, sizeof(GemmSmem<T>)))
+            if(j0 == 0 && !set_smem(k, sizeof(GemmSmem<T>)))
                 return rocblas_status_internal_error;
             const int tm = (below + 63) / 64, tn = (right + 63) / 64;
             RSB_LOG_KERNEL("getrf_gemm_kernel");

@@ -15,15 +15,12 @@
 
 #include "common.cuh"
 #include "lu_cta.cuh" // fma2, WarpTileTF32
-#include "vbatched.h"
 
 namespace rsb {
 
 constexpr int BLK_NB = 64;
 
-// The members of one call: a uniform batch (v.n == nullptr) or a variable-size one (members
-// in the order of v.order, largest first; those of at most VB_SMALL rows and the invalid ones
-// are left out).
+// the members of one call
 template <typename T>
 struct LuBatch
 {
@@ -33,8 +30,6 @@ struct LuBatch
     int64_t strideP;
     int* info;
     Gate gate;
-    VbArgs v;
-    T* const* vA;
 };
 
 template <typename T>
@@ -49,19 +44,6 @@ struct LuMember
 template <typename T>
 __device__ __forceinline__ bool lu_member(const LuBatch<T>& L, int64_t i, LuMember<T>& M)
 {
-    if(L.v.n)
-    {
-        const int b = L.v.order[i];
-        const int n = L.v.n[b];
-        if(n <= VB_SMALL || !vb_valid(L.v, b))
-            return false;
-        M.a = L.vA[b];
-        M.lda = L.v.lda[b];
-        M.m = M.n = n;
-        M.piv = L.v.ipiv[b];
-        M.info = L.v.info + b;
-        return true;
-    }
     if(L.gate.skip(i))
         return false;
     M.a = L.A.at(i);
@@ -244,12 +226,12 @@ struct PanelShape
 };
 constexpr int PANEL_LDU = BLK_NB + 4;
 
-template <typename T, int NB, int S>
+template <typename T, int NB, int S, bool CL>
 struct PanelSmem
 {
     T P[NB][PanelShape<T, S>::LDP]; // finished (and the current group's) columns, by row slot
     T R[8][PANEL_LDU];              // the group's pivot rows right of the group, then U
-    T U[8][PANEL_LDU];              // U of the group (written apart from R only in a cluster)
+    T U[CL ? 8 : 1][PANEL_LDU];     // (cluster) U of the group; else it takes the place of R
     T L8[8][8];                     // the pivot rows within the group
     PanelRec<T> rec[2][16];         // candidates, double-buffered by column parity; [.][rank, warp]
     PanelRec<T> mine[2];
@@ -290,7 +272,7 @@ struct PanelLabels
 // Time of one 64-column FP64 panel alone on an SM: 64 rows (S = 2) 36 us, 128 rows 33 us; 256
 // rows took 58 us with one warp of 8 rows a lane, which is why they have two.
 template <typename T, int NB, int SC, bool PIVOT, bool CL>
-__device__ __forceinline__ void panel_group(PanelSmem<T, NB, SC>& sm,
+__device__ __forceinline__ void panel_group(PanelSmem<T, NB, SC, CL>& sm,
                                             PanelLabels<PanelShape<T, SC>::FS>& st, int f, int c0,
                                             int gb, int j0, int rank, int nrank, int wait_limit)
 {
@@ -639,28 +621,29 @@ struct PanelUpdate<float, NB>
     }
 };
 
-// The panel at (j0, j0): rows j0..m-1, jb = min(NB, min(m, n) - j0) columns.  The row warps
+// The panel at (j0, j0): rows j0..m-1 (at most 32 S a CTA), jb = min(NB, min(m, n) - j0) columns.  The row warps
 // hold the columns right of the current group of 8 in registers, in tensor-accumulator
-// layout; the group itself is factored by one warp from shared memory (panel_group).  Then
+// layout; the group itself is factored by one warp, or two for 256 rows, from shared memory
+// (panel_group).  Then
 // the group's pivot rows are published, U of the group is formed (one thread per column, 8 x
 // 8 unit-lower substitution) and the rows take the rank-8 update: first the next group's
 // columns, which go to shared memory, then, while that group is being factored, the
 // others.  The update moves chunk ch to register chunk ch - 1, so that the group loop is one
 // copy of the code.
 // CL: a cluster of CTAs, each with 32 * S of the rows; candidates and pivot rows cross it
-// through distributed shared memory.  Members of a variable-size batch are taken when their
-// row count lies in (rows_lo, rows_hi].
+// through distributed shared memory.
 template <typename T, int NB, int S, bool PIVOT, bool CL>
 __global__ void __launch_bounds__(PanelShape<T, S>::NT,
                                   S <= 2   ? (sizeof(T) == 8 ? 4 : 6)
                                   : S <= 4 ? (sizeof(T) == 8 ? 2 : 3)
                                            : (sizeof(T) == 8 || CL ? 1 : 2))
-    lu_panel_kernel(LuBatch<T> L, int j0, int rows_lo, int rows_hi, int wait_limit)
+    lu_panel_kernel(LuBatch<T> L, int j0, int wait_limit)
 {
     using SH = PanelShape<T, S>;
     constexpr int RT = SH::RT, NT = SH::NT, NC = NB / 8 - 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    PanelSmem<T, NB, S>& sm = *reinterpret_cast<PanelSmem<T, NB, S>*>(smem_raw);
+    using Smem = PanelSmem<T, NB, S, CL>;
+    Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     int nrank = 1, rank = 0;
     if(CL)
     {
@@ -671,8 +654,6 @@ __global__ void __launch_bounds__(PanelShape<T, S>::NT,
     if(!lu_member(L, blockIdx.x / nrank, M) || (j0 > 0 && lu_gave_up(L, M)))
         return;
     const int mn = min(M.m, M.n), mp = M.m - j0;
-    if(j0 >= mn || mp <= rows_lo || mp > rows_hi)
-        return;
     const int jb = min(NB, mn - j0);
     const int rbase = rank * RT; // this CTA's rows of the panel
     const int mc = max(0, min(RT, mp - rbase));
@@ -900,6 +881,48 @@ struct TrsmSmem
     int piv[BLK_NB], src[BLK_NB], dst[BLK_NB];
 };
 
+// rows ib..ib+15 of 16 columns -= L(ib.., 0..ib-1) X as a 16 x 16 tensor tile of one warp;
+// L [k][i], x [column][k]
+__device__ __forceinline__ void trsm_tile(const double (*L)[BLK_NB + 4], double* x, int ib)
+{
+    constexpr int LD = BLK_NB + 1;
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    double acc[2][2][2];
+#pragma unroll
+    for(int i = 0; i < 2; ++i)
+#pragma unroll
+        for(int j = 0; j < 2; ++j)
+#pragma unroll
+            for(int e = 0; e < 2; ++e)
+                acc[i][j][e] = x[(8 * j + 2 * q + e) * LD + ib + 8 * i + g];
+#pragma unroll 4
+    for(int k = 0; k < ib; k += 4)
+    {
+        double a[2], b[2];
+#pragma unroll
+        for(int i = 0; i < 2; ++i)
+        {
+            a[i] = -L[k + q][ib + 8 * i + g];
+            b[i] = x[(8 * i + g) * LD + k + q];
+        }
+#pragma unroll
+        for(int i = 0; i < 2; ++i)
+#pragma unroll
+            for(int j = 0; j < 2; ++j)
+                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
+                             "{%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                             : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
+                             : "d"(a[i]), "d"(b[j]));
+    }
+#pragma unroll
+    for(int i = 0; i < 2; ++i)
+#pragma unroll
+        for(int j = 0; j < 2; ++j)
+#pragma unroll
+            for(int e = 0; e < 2; ++e)
+                x[(8 * j + 2 * q + e) * LD + ib + 8 * i + g] = acc[i][j][e];
+}
+
 template <typename T, bool PIVOT>
 __global__ void __launch_bounds__(TRSM_NT, sizeof(T) == 8 ? 3 : 5)
     lu_swap_trsm_kernel(LuBatch<T> L, int j0, int chunks)
@@ -912,8 +935,6 @@ __global__ void __launch_bounds__(TRSM_NT, sizeof(T) == 8 ? 3 : 5)
         return;
     const int jb = min(NB, min(M.m, M.n) - j0);
     const int cfirst = j0 + jb + (blockIdx.x % chunks) * CW;
-    if(jb <= 0 || cfirst >= M.n)
-        return;
     const int ncol = min(CW, M.n - cfirst);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for(int e = tid; e < NB * NB; e += NT)
@@ -999,46 +1020,8 @@ __global__ void __launch_bounds__(TRSM_NT, sizeof(T) == 8 ? 3 : 5)
     {
         if constexpr(sizeof(T) == 8)
         {
-            // rows ib..ib+15 -= L11(ib.., 0..ib-1) X: 16 x 16 tensor tiles, one per warp
             if(ib > 0 && warp * 16 < ncol)
-            {
-                const int g = lane >> 2, q = lane & 3;
-                double* x = &sm.X[warp * 16][0];
-                double acc[2][2][2];
-#pragma unroll
-                for(int i = 0; i < 2; ++i)
-#pragma unroll
-                    for(int j = 0; j < 2; ++j)
-#pragma unroll
-                        for(int e = 0; e < 2; ++e)
-                            acc[i][j][e] = x[(8 * j + 2 * q + e) * (NB + 1) + ib + 8 * i + g];
-#pragma unroll 4
-                for(int k = 0; k < ib; k += 4)
-                {
-                    double a[2], b[2];
-#pragma unroll
-                    for(int i = 0; i < 2; ++i)
-                    {
-                        a[i] = -sm.L[k + q][ib + 8 * i + g];
-                        b[i] = x[(8 * i + g) * (NB + 1) + k + q];
-                    }
-#pragma unroll
-                    for(int i = 0; i < 2; ++i)
-#pragma unroll
-                        for(int j = 0; j < 2; ++j)
-                            asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 "
-                                         "{%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                                         : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
-                                         : "d"(a[i]), "d"(b[j]));
-                }
-#pragma unroll
-                for(int i = 0; i < 2; ++i)
-#pragma unroll
-                    for(int j = 0; j < 2; ++j)
-#pragma unroll
-                        for(int e = 0; e < 2; ++e)
-                            x[(8 * j + 2 * q + e) * (NB + 1) + ib + 8 * i + g] = acc[i][j][e];
-            }
+                trsm_tile(sm.L, &sm.X[warp * 16][0], ib);
             __syncthreads();
         }
         if(tid < ncol)
@@ -1206,13 +1189,12 @@ struct GemmSmem
 };
 
 template <typename T, bool TC, bool FULL>
-__device__ __forceinline__ void gemm_tile(GemmSmem<T>& sm, const LuMember<T>& M, int j0, int jb,
-                                          int r0, int c0, int nr, int nc)
+__device__ __forceinline__ void gemm_tile(GemmSmem<T>& sm, const LuMember<T>& M, int j0, int r0,
+                                          int c0, int nr, int nc)
 {
     using Tile = GemmTile<T, TC>;
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int kk = FULL ? 64 : (jb + 7) & ~7;
-    // operands; rows, columns and k outside the member are zero
+    // operands; rows and columns outside the member are zero
     if constexpr(FULL)
     {
         constexpr int V = 16 / sizeof(T), PER = 64 / V; // vectors of a column
@@ -1234,10 +1216,10 @@ __device__ __forceinline__ void gemm_tile(GemmSmem<T>& sm, const LuMember<T>& M,
     }
     else
     {
-        for(int e = tid; e < kk * 64; e += 128)
+        for(int e = tid; e < 64 * 64; e += 128)
         {
             const int i = e & 63, k = e >> 6;
-            if(i < nr && k < jb)
+            if(i < nr)
                 cp_async(&sm.A[k][i], &RSB_AT(M.a, r0 + i, j0 + k, M.lda, M.m, M.n));
             else
                 sm.A[k][i] = T(0);
@@ -1251,7 +1233,7 @@ __device__ __forceinline__ void gemm_tile(GemmSmem<T>& sm, const LuMember<T>& M,
             const int k = Tile::B_BY_COL ? (e & 63) : ((e & 7) | ((e >> 4) & 0x38));
             const int c = Tile::B_BY_COL ? (e >> 6) : (((e >> 3) & 15) | ((e >> 6) & 0x30));
             T* d = Tile::B_BY_COL ? &sm.B[c][k] : &sm.B[k][c];
-            if(FULL || (c < nc && k < jb))
+            if(FULL || c < nc)
                 cp_async(d, &RSB_AT(M.a, j0 + k, c0 + c, M.lda, M.m, M.n));
             else
                 *d = T(0);
@@ -1269,7 +1251,7 @@ __device__ __forceinline__ void gemm_tile(GemmSmem<T>& sm, const LuMember<T>& M,
     __syncthreads();
     if(live)
     {
-        w.mma(&sm.A[0][0], &sm.B[0][0], wr, wc, kk);
+        w.mma(&sm.A[0][0], &sm.B[0][0], wr, wc, BLK_NB);
         w.each([&](int r, int c, auto& v) {
             if(FULL || (wr + r < nr && wc + c < nc))
                 RSB_AT(M.a, r0 + wr + r, c0 + wc + c, M.lda, M.m, M.n) = -v;
@@ -1277,8 +1259,8 @@ __device__ __forceinline__ void gemm_tile(GemmSmem<T>& sm, const LuMember<T>& M,
     }
 }
 
-// A22 -= L21 U12 for the panel at j0: one CTA of four warps per 64 x 64 tile, K = jb <= 64 in
-// one stage.  The tile of A22 is loaded (negated) into the accumulators while cp.async brings
+// A22 -= L21 U12 for the panel at j0: one CTA of four warps per 64 x 64 tile, K = 64 in one
+// stage (a panel with fewer columns has no rows below or no columns right of it).  The tile of A22 is loaded (negated) into the accumulators while cp.async brings
 // the operands in; several CTAs per SM overlap one tile's loads with another's products.
 template <typename T, bool TC>
 __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 3 : 4)
@@ -1290,21 +1272,18 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 3 : 4)
     LuMember<T> M;
     if(!lu_member(L, blockIdx.x / tiles, M) || lu_gave_up(L, M))
         return;
-    const int jb = min(NB, min(M.m, M.n) - j0);
     const int t = blockIdx.x % tiles;
-    const int r0 = j0 + jb + (t % tiles_m) * 64, c0 = j0 + jb + (t / tiles_m) * 64;
-    if(jb <= 0 || r0 >= M.m || c0 >= M.n)
-        return;
+    const int r0 = j0 + NB + (t % tiles_m) * 64, c0 = j0 + NB + (t / tiles_m) * 64;
     const int nr = min(64, M.m - r0), nc = min(64, M.n - c0);
     // whole tiles of 16-byte aligned columns (one branch per CTA): no bounds, 16-byte copies
-    const bool full = nr == 64 && nc == 64 && jb == 64
+    const bool full = nr == 64 && nc == 64
                       && ((reinterpret_cast<uintptr_t>(M.a) | ((uintptr_t)M.lda * sizeof(T))
                            | ((uintptr_t)r0 * sizeof(T)))
                           & 15) == 0;
     if(full)
-        gemm_tile<T, TC, true>(sm, M, j0, jb, r0, c0, nr, nc);
+        gemm_tile<T, TC, true>(sm, M, j0, r0, c0, nr, nc);
     else
-        gemm_tile<T, TC, false>(sm, M, j0, jb, r0, c0, nr, nc);
+        gemm_tile<T, TC, false>(sm, M, j0, r0, c0, nr, nc);
 }
 
 // ---------------------------------------------------------------------------- L's rows
@@ -1331,8 +1310,6 @@ __global__ void __launch_bounds__(LEFT_NT)
     const int c0 = (t / PARTS) * NB + (t % PARTS) * LEFT_COLS;
     const int r0 = (t / PARTS + 1) * NB; // first row the later panels may move
     const int mn = min(M.m, M.n), rows = M.m - r0;
-    if(r0 >= mn)
-        return;
     const int tid = threadIdx.x;
     for(int q = tid; q < rows; q += LEFT_NT)
         perm[q] = s[q] = q;

@@ -6,7 +6,7 @@
 
 namespace rsb {
 
-// LU of the members of L (their largest dimensions m x n, m <= 2048); bc members
+// LU of the bc members of L (m x n, m <= 2048)
 template <typename T>
 rocblas_status launch_lu_blk(cudaStream_t s, const LuBatch<T>& L, int m, int n, int bc,
                              bool pivot, bool tc);

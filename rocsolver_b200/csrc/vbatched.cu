@@ -20,11 +20,38 @@
 #include "lu_cta.cuh"
 #include "lu_small.cuh"
 #include "trsv.cuh"
-#include "vbatched.h"
 
 namespace rsb {
 
+constexpr int VB_SMALL = 32; // members with n <= VB_SMALL use the warp path
 constexpr int VB_WARPS = 8;    // CTA = 8 warps = 256 threads
+
+struct VbArgs
+{
+    int bc, max_n, max_nrhs, mode; // mode: 0 gesv, 1 getrf, 2 getrs
+    const int* n;
+    const int* nrhs;
+    const int* lda;
+    const int* ldb;
+    int* const* ipiv;
+    int* info;
+    int* order;    // [bc]
+    int* counters; // [0] big cursor, [1] small cursor, [2] number of big members
+};
+
+__device__ __forceinline__ bool vb_valid(const VbArgs& v, int b)
+{
+    const int n = v.n[b];
+    if(n < 0 || n > v.max_n || v.lda[b] < max(1, n))
+        return false;
+    if(v.mode != 1)
+    {
+        const int r = v.nrhs[b];
+        if(r < 0 || r > v.max_nrhs || v.ldb[b] < max(1, n))
+            return false;
+    }
+    return true;
+}
 
 __global__ void __launch_bounds__(1024) vb_plan_kernel(VbArgs v)
 {
