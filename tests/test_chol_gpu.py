@@ -92,6 +92,40 @@ def test_potrf_spd(handle, n, lower, dtype):
     check_potrf(A, C, info, lower)
 
 
+@pytest.mark.parametrize("n,lower,dtype", [(1025, True, np.float64), (1025, False, np.float64),
+                                           (1025, True, np.float32), (1025, False, np.float32),
+                                           (2048, True, np.float64), (2048, False, np.float32)])
+def test_potrf_large(handle, n, lower, dtype):
+    """Up to the largest order, odd leading dimensions; a member that fails in a late panel."""
+    A = spd_gram(n, 2, seed=n).astype(dtype)
+    A[1, n - 70, n - 70] = -1.0
+    C, info, _ = gpu_potrf(handle, A, lower, lda=n + 1 + (n % 2))
+    assert info[0] == 0 and 64 < info[1] <= n - 69
+    check_potrf(A, C, info, lower)
+
+
+@pytest.mark.parametrize("n,k", [(100, 70), (200, 64), (200, 190), (600, 513)])
+@pytest.mark.parametrize("lower", [True, False])
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_potrf_nan_and_inf_beyond_the_first_block(handle, n, k, lower, value):
+    """A NaN or -infinity on the diagonal stops the member there; +infinity is a pivot like any
+    other, whose column is zero below, and the columns before it are the oracle's."""
+    A = spd_gram(n, 2, seed=n + k)
+    A[1, k, k] = value
+    C, info, _ = gpu_potrf(handle, A, lower)
+    oC, oinfo = oracle_potrf(A, lower)
+    np.testing.assert_array_equal(info, oinfo)
+    tri = (lambda x: np.tril(x)) if lower else (lambda x: np.triu(x).T)
+    G, O = tri(C[1]), tri(oC[1])
+    scale = np.abs(O[:k, :k]).max()
+    assert np.abs(G[:k, :k] - O[:k, :k]).max() <= 4 * n * eps_of(np.float64) * scale
+    if value == np.inf:
+        assert np.isinf(G[k, k]) and not G[k + 1:, k].any()
+    else:
+        assert info[1] == k + 1 and (np.isnan(G[k, k]) if np.isnan(value) else G[k, k] == value)
+    check_potrf(A[:1], C[:1], info[:1], lower)
+
+
 def gpu_potrs(handle, C, B, lower, batched=False):
     bc, n, _ = C.shape
     nrhs = B.shape[2]

@@ -1,13 +1,17 @@
 """The blocked LU (64-column steps in separate launches: panel, interchanges with U12, trailing
 update, L's rows) against the oracle at the sizes where it can go wrong: one column more or
 less than a panel, every CTA row count and cluster size of the panel kernel, rectangular
-members, padded and odd leading dimensions, tied pivots, infinities and NaN."""
+members, padded and odd leading dimensions, tied pivots, infinities and NaN.  With a few
+members the built-in choice takes it for FP64 above 512 rows (whose later panels have every
+smaller row count) and for FP32 at most sizes; the FP64 cases of up to 512 rows check the same
+properties of the CTA kernels that run there."""
 import numpy as np
 import pytest
 
 import rocsolver_b200 as rs
-from tests.gpu_util import GpuHandle
-from tests.refcases import uniform_general
+from tests.gpu_util import GpuHandle, dev, host, ptr
+from tests.norms import lu_backward_error
+from tests.refcases import from_colmajor, to_colmajor, uniform_general
 from tests.test_lu_gpu import check_getrf, gpu_getrf, oracle_getrf
 
 pytestmark = pytest.mark.gpu
@@ -22,7 +26,7 @@ def handle():
 
 @pytest.fixture(autouse=True)
 def no_table():
-    """Without tuning entries every m > 32 takes the blocked path."""
+    """Without tuning entries the built-in choice runs."""
     old = rs.tuning_table()
     assert rs.set_tuning_table("") == rs.SUCCESS
     yield
@@ -41,6 +45,61 @@ def test_blocked_getrf(handle, m, n, pad):
     check_getrf(A, LU, ipiv, info)
 
 
+@pytest.mark.parametrize("m,n", [(513, 513), (577, 577), (640, 640), (600, 1300), (700, 400)])
+@pytest.mark.parametrize("pad", [0, 3])
+def test_blocked_dgetrf_above_512_rows(handle, m, n, pad):
+    """A last panel of 1, 1, 64 and 24 columns and a wide member, FP64."""
+    A = uniform_general(m, n, 2, seed=m * 7 + n)
+    LU, ipiv, info, _ = gpu_getrf(handle, A, lda=m + pad)
+    check_getrf(A, LU, ipiv, info)
+
+
+def _dominant32(m, n, bc, seed):
+    """uniform[-1, 1] with one large entry per column (the rows drawn at random), so that FP32
+    rounding decides no pivot"""
+    A = uniform_general(m, n, bc, seed=seed)
+    rng = np.random.default_rng(seed)
+    for b in range(bc):
+        k = min(m, n)
+        A[b, rng.permutation(m)[:k], np.arange(k)] += 6 + 0.2 * n
+    return A.astype(np.float32)
+
+
+@pytest.mark.parametrize("m,n", [(20, 100), (32, 33), (33, 33), (64, 64), (33, 100), (64, 130),
+                                 (97, 97), (127, 127), (128, 300), (161, 161), (256, 256),
+                                 (257, 257), (320, 320), (512, 512), (513, 300), (1025, 600)])
+@pytest.mark.parametrize("pad", [0, 3])
+def test_blocked_sgetrf_sizes(handle, m, n, pad):
+    A = _dominant32(m, n, 2, seed=m * 7 + n)
+    LU, ipiv, info, _ = gpu_getrf(handle, A, lda=m + pad)
+    check_getrf(A, LU, ipiv, info)
+
+
+@pytest.mark.parametrize("prec,n", [("d", 1500), ("d", 2048), ("s", 2048), ("t", 2048)])
+def test_blocked_getrf_large_square(handle, prec, n):
+    """The longest trailing sweep: 24 and 32 panels, clusters of 8 down to single CTAs, L's rows
+    with the most interchanges, an odd leading dimension."""
+    if prec == "d":
+        A = uniform_general(n, n, 1, seed=n)
+    else:
+        A = _dominant32(n, n, 1, seed=n)
+    if prec != "t":
+        LU, ipiv, info, _ = gpu_getrf(handle, A, lda=n + 1)
+        check_getrf(A, LU, ipiv, info)
+        return
+    dA = dev(to_colmajor(A, n + 1))
+    dP, dI = dev(np.zeros(n, np.int32)), dev(np.full(1, -7, np.int32))
+    st = rs.call("rocsolver_sgetrf_tf32_strided_batched", handle, n, n, ptr(dA), n + 1,
+                 (n + 1) * n, ptr(dP), n, ptr(dI), 1)
+    assert st == rs.SUCCESS
+    LU = from_colmajor(host(dA), 1, n, n, n + 1, (n + 1) * n)[0].astype(np.float64)
+    _, oipiv, oinfo = oracle_getrf(A)
+    np.testing.assert_array_equal(host(dI), oinfo)
+    np.testing.assert_array_equal(host(dP), oipiv[0])
+    be = lu_backward_error(A[0].astype(np.float64), LU, host(dP))
+    assert be / (n * np.finfo(np.float32).eps) < 10
+
+
 @pytest.mark.parametrize("m,n", [(65, 65), (200, 330), (600, 600)])
 def test_blocked_getrf_npvt_and_pointer_batch(handle, m, n):
     A = uniform_general(m, n, 2, seed=m) + 2 * max(m, n) * np.eye(m, n)
@@ -51,11 +110,12 @@ def test_blocked_getrf_npvt_and_pointer_batch(handle, m, n):
 
 
 @pytest.mark.parametrize("n", [64, 70, 300, 520])
-def test_blocked_getrf_ties_and_zero_columns(handle, n):
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_blocked_getrf_ties_and_zero_columns(handle, n, dtype):
     """Entries -1, 0, 1: columns full of equal candidates (the smallest row position wins, in
     the lane, across lanes, warps and CTAs); a zero column sets info."""
     rng = np.random.default_rng(n)
-    A = rng.integers(-1, 2, (3, n, n)).astype(np.float64)
+    A = rng.integers(-1, 2, (3, n, n)).astype(dtype)
     A[1][:, n // 2] = 0.0
     LU, ipiv, info, _ = gpu_getrf(handle, A)
     oLU, oipiv, oinfo = oracle_getrf(A)
@@ -65,22 +125,25 @@ def test_blocked_getrf_ties_and_zero_columns(handle, n):
     np.testing.assert_array_equal(ipiv.reshape(3, n)[:, :k], oipiv[:, :k])
     # and the factors multiply back to the permuted matrix
     for b in range(3):
-        L = np.tril(LU[b], -1) + np.eye(n)
-        R = L @ np.triu(LU[b])
+        F = LU[b].astype(np.float64)
+        L = np.tril(F, -1) + np.eye(n)
+        R = L @ np.triu(F)
         P = A[b].copy()
         for i, p in enumerate(ipiv.reshape(3, n)[b]):
             P[[i, p - 1]] = P[[p - 1, i]]
-        assert np.abs(R - P).max() <= n * np.finfo(float).eps * np.abs(L).sum(1).max() \
-            * np.abs(LU[b]).max()
+        assert np.abs(R - P).max() <= n * np.finfo(dtype).eps * np.abs(L).sum(1).max() \
+            * np.abs(F).max()
     assert info[1] == oinfo[1] != 0
 
 
-@pytest.mark.parametrize("n", [64, 200, 400])
-def test_blocked_getrf_nan_and_inf(handle, n):
+@pytest.mark.parametrize("n,dtype", [(64, np.float64), (200, np.float64), (400, np.float64),
+                                     (600, np.float64), (64, np.float32), (256, np.float32),
+                                     (400, np.float32), (600, np.float32)])
+def test_blocked_getrf_nan_and_inf(handle, n, dtype):
     """A NaN below the diagonal never wins the search, a NaN on it is kept; an infinity wins;
     entries that they do not reach stay finite (compared with the oracle up to the column
     where the first of them is eliminated)."""
-    A = uniform_general(n, n, 3, seed=n)
+    A = uniform_general(n, n, 3, seed=n).astype(dtype)
     A[0][n - 1, 0] = np.nan
     A[1][0, 0] = np.nan
     A[2][n // 2, 1] = np.inf
@@ -89,7 +152,8 @@ def test_blocked_getrf_nan_and_inf(handle, n):
     np.testing.assert_array_equal(ipiv.reshape(3, n)[:, :2], oipiv[:, :2])
     for b in range(3):
         np.testing.assert_array_equal(np.isnan(LU[b][:, :2]), np.isnan(oLU[b][:, :2]))
-    np.testing.assert_allclose(LU[0][:1], oLU[0][:1], rtol=1e-13)
+    # the first row of U is the pivot row as it was
+    np.testing.assert_array_equal(LU[0][:1], oLU[0][:1])
 
 
 @pytest.mark.parametrize("m,n", [(64, 64), (129, 129), (300, 300), (520, 130), (1030, 70)])
