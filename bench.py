@@ -220,14 +220,17 @@ def build_workload(name, torch, rs, dev, handle):
             w.config["workload"] = ("dsgesv_strided_batched (FP32 LU + FP64 IR, <=10 iters, FP64 "
                                     "fallback) vs plain dgetrf+dgetrs, n=256, batch=2048, nrhs=1, "
                                     "cond log-uniform [1e1,1e6]")
-            w.dominant = ("getrf_cta_kernel<float, 128, 2, 32, TF32> (FP32 LU with split-TF32 "
-                          "tensor-core trailing updates inside dsgesv)")
-            # 714.1 MB per 512 members from `ncu --set full --clock-control none -c 1
-            # -k regex:getrf_cta python -m rocsolver_b200.demo --case dsgesv --n 256
-            # --batch 512 --reps 1`
-            w.traffic_per_unit = 714073856 / 512
+            w.dominant = ("lu_panel, lu_swap_trsm, lu_gemm and lu_left kernels (the blocked FP32 LU "
+                          "with split-TF32 tensor-core trailing updates inside dsgesv)")
+            # DRAM bytes of its 11 launches per member: 3272.8 MB per 2048 members from
+            # `ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none
+            # -k regex:lu_ python -m rocsolver_b200.demo --case sgetrf_tf32 --n 256
+            # --batch 2048 --reps 1`
+            w.traffic_per_unit = 3272800000 / 2048
             w.limiter = "latency: the per-column pivot chain (TF32 tensor fraction beside it)"
-            w.launches_per_step = 6
+            # conversion; 4 panels, 3 interchanges with U12, 3 updates, 1 for L's rows;
+            # refinement; the gated FP64 LU, copy and solve
+            w.launches_per_step = 1 + (4 + 3 + 3 + 1) + 1 + 3
     elif name == "getrf_n32":
         n, bc, nrhs = 32, 1000, 1
         rng = np.random.default_rng(0)
