@@ -1899,8 +1899,8 @@ ROCSOLVER_EXPORT rocblas_status rocsolver_dgesv_vbatched_noalloc(rocblas_handle 
  * uses the s entries; fold = 2 in a t entry runs its trailing updates on the tcgen05 tensor
  * cores).  It is written by the autotuner (python -m rocsolver_b200.tune) and read when the first
  * handle is created, from $ROCSOLVER_B200_TUNING or else tuning_b200.txt beside the
- * library.  Entries that name an unavailable configuration fall back to the built-in
- * choice; results do not depend on the table, only speed does. */
+ * library.  Entries that name an unavailable configuration (zeros do) fall back to the
+ * built-in choice; apart from rounding, results do not depend on the table. */
 ROCSOLVER_EXPORT rocblas_status rocsolver_b200_tuning_set(const char* text);   /* replace */
 ROCSOLVER_EXPORT rocblas_status rocsolver_b200_tuning_load(const char* path);  /* from file */
 /* Writes the active table (NUL-terminated, truncated to len) and returns its full size

@@ -7,6 +7,11 @@
 // upper case (A = U' U) is the same on the transposed view; both read and write along the
 // stored columns.  Members whose info is set are left alone, except that a member that failed
 // in this step still gets the finished columns of its panel (LAPACK potf2).
+//
+// potrf alone against one CTA per member with a barrier per column: FP32 n = 200 x 1500 0.56 ms
+// (4.2), of it updates 0.25, panels 0.16 and diagonal blocks 0.15; FP64 n = 128 x 4882 0.62 (9.2),
+// n = 65 x 1 0.040 (0.093), n = 2048 x 16 4.3 (358).  One launch of the diagonal block is a serial
+// chain of 64 columns, which is what small batches wait for.
 #pragma once
 
 #include "lu_blk.cuh" // GemmTile, cp.async helpers

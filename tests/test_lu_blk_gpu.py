@@ -245,3 +245,52 @@ def test_cluster_wait_that_runs_out():
                        capture_output=True, text=True, timeout=600, cwd=root)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
     assert "waits done" in r.stdout
+
+
+@pytest.mark.parametrize("fn,prec,n,bc", [("getrf", "d", 600, 2), ("getrf", "s", 200, 3),
+                                          ("getrf", "s", 65, 3), ("potrf", "d", 200, 3)])
+def test_blocked_calls_in_a_captured_graph(fn, prec, n, bc):
+    """The launches of a blocked call captured in a CUDA graph: the replay on other values gives
+    the direct call's bits."""
+    import torch
+    dt = torch.float64 if prec == "d" else torch.float32
+    g = torch.Generator(device="cuda").manual_seed(n)
+    A0 = torch.rand(2, bc, n, n, dtype=dt, device="cuda", generator=g)
+    A0 = A0 + A0.transpose(2, 3) + 2 * n * torch.eye(n, dtype=dt, device="cuda")
+    src, A = A0[0].clone(), torch.empty_like(A0[0])
+    ipiv = torch.zeros(bc, n, dtype=torch.int32, device="cuda")
+    info = torch.zeros(bc, dtype=torch.int32, device="cuda")
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    h = rs.Handle(stream.cuda_stream)
+
+    def call():
+        A.copy_(src)
+        if fn == "getrf":
+            st = rs.call(f"rocsolver_{prec}getrf_strided_batched", h.value, n, n, ptr(A), n, n * n,
+                         ptr(ipiv), n, ptr(info), bc)
+        else:
+            st = rs.call(f"rocsolver_{prec}potrf_strided_batched", h.value, rs.FILL_UPPER, n,
+                         ptr(A), n, n * n, ptr(info), bc)
+        rs.check(st, fn)
+
+    try:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(stream):
+            call()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            call()
+        src.copy_(A0[1])
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        got = (A.clone(), ipiv.clone(), info.clone())
+        with torch.cuda.stream(stream):
+            call()
+        torch.cuda.synchronize()
+        for x, y in zip(got, (A, ipiv, info)):
+            assert torch.equal(x, y)
+        assert not info.any()
+    finally:
+        h.close()
